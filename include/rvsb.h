@@ -414,10 +414,9 @@ rvsb_status rvsb_batch_reserve(rvsb_batch* batch, int max_width, int max_height)
 rvsb_status rvsb_batch_set_graphs(rvsb_batch* batch, int enable);
 /* Raster autotuner (default off): the first batch of each new shape (batch
  * size bucket, largest input set and output, projections) is run once with
- * every raster variant -- tile size 32x32 or 64x32, views per shared
- * z-buffer group, the stretched-triangle threshold, threads per tile (512 or
- * 1024) and whether triangles whose candidate box holds up to 32 pixels
- * take the one-lane-per-pixel medium path -- and the fastest is kept for that shape.
+ * every raster variant -- quad rows per warp and the candidate-pixel count
+ * above which a triangle is rasterised by a whole warp instead of one lane --
+ * and the fastest is kept for that shape.
  * All variants give identical outputs. */
 rvsb_status rvsb_batch_set_autotune(rvsb_batch* batch, int enable);
 /* Use one raster variant (0 .. 7) for every call, or -1 for the default or
@@ -477,9 +476,11 @@ void rvsb_server_destroy(rvsb_server* server);
 
 /* Per-stage timing with CUDA events recorded on the launch stream (the
  * per-stage timers that replace the reference's whole-run clock(),
- * rvs/src/view_synthesis.cpp:149-166).  Stages: 0 warp, 1 bin, 2 raster
- * (with the resolve, blend and quantisation of every tile), 3 inpaint,
- * 4 whole synthesis. */
+ * rvs/src/view_synthesis.cpp:149-166).  Stages: 0 warp (with the
+ * rasterisation of the warped triangles into the z-buffers), 1 bin (the
+ * listed large triangles), 2 raster (resolve, blend and quantisation; for
+ * more than four input views also the stages 0 and 1 of the view groups
+ * after the first), 3 inpaint, 4 whole synthesis. */
 #define RVSB_NUM_STAGES 5
 rvsb_status rvsb_scene_set_profiling(rvsb_scene* scene, int enable);
 /* Milliseconds per stage of the most recent profiled synthesis; call after

@@ -5,20 +5,9 @@
 
 namespace rvsb {
 
-// Tiling constants.  A binning block is BLOCK_W x BLOCK_H quads of an input
-// view (each quad = two triangles, transform.cpp:159-176); an output tile
-// (its size is chosen per batch among the raster variants) holds 64-bit
-// z-buffers in shared memory and is processed by one CTA of the variant's
-// thread count (TILE_THREADS unless the variant names another).
-constexpr int BLOCK_W = 8;
-constexpr int BLOCK_H = 4;
-// Vertex tile of the warp kernel (WARP_TILE x WARP_TILE input pixels per CTA),
-// also the unit of the ERP input culling tables.
+// Vertex tile of the ERP input culling tables (WARP_TILE x WARP_TILE input
+// pixels).
 constexpr int WARP_TILE = 32;
-constexpr int TILE_THREADS = 512;
-// Smallest tile of any raster variant (sizes the bin arrays).
-constexpr int MIN_TILE_W = 32;
-constexpr int MIN_TILE_H = 32;
 
 // Per input view parameters of one synthesis (device copy in a table).
 struct DevView {
@@ -47,8 +36,7 @@ struct DevView {
     const float2* tile_depth;
     const uint64_t* color;                // h*w decoded colour: Y | 4U << 18 | 4V << 36
     float4* vert;                         // h*w warped vertices (u, v, z, 0)
-    int4* bbox;                           // per binning block: x0, y0, x1, y1 (x0 > x1: empty)
-    int nbx, nby;                         // binning blocks
+    unsigned long long* z;                // wo*ho fragment keys (shared by the views of one group each)
     int tri_shift;                        // triangle index = i << tri_shift | j << 2 | t
     int pad;
 };
@@ -81,10 +69,7 @@ struct DevTarget {
     float precision;
     int rs_area;                          // the resize is an exact 2x reduction (area mean)
     double rs_scale_x, rs_scale_y;        // raster size / output size (double), bilinear
-    int tile_wl, tile_hl;                 // log2 of the tile width and height
-    int ntx, nty;                         // output tiles
     int n_views;
-    int bin_capacity;
 };
 
 // Largest number of input views of one synthesis.
@@ -92,11 +77,10 @@ constexpr int MAX_VIEWS = 16;
 
 // Status words written by the kernels (device memory, reset per call).
 struct DevStatus {
-    int bin_total;      // number of (tile, view, block) entries
-    int bin_overflow;   // 1 when bin_total exceeded the list capacity
+    int n_large;        // large triangles entered in the list (may exceed its capacity)
     int hole_x0, hole_y0, hole_x1, hole_y1;   // bounding box of holes (x0 > x1: none)
     int n_holes;
-    int pad;
+    int pad[2];
 };
 
 // Optional intermediate outputs (device pointers, may be null).
@@ -151,17 +135,18 @@ struct MsPtrs {
 // Device buffers of one slot's workspace.
 struct SlotBuffers {
     DevStatus* status;   // 1 entry
-    int* counts;         // ntiles * n_views
-    int* offsets;        // ntiles * n_views
-    int* cursor;         // ntiles * n_views
-    int* list;           // bin list, `capacity` entries
-    int capacity;
+    uint4* large;        // large triangles of the view group, `large_capacity` entries
+    int large_capacity;
     int pad;
+    // Running blend between view groups: (c0, c1) and (c2, weight sum) per
+    // pixel; they share the memory of the last scan buffer and the codes,
+    // which are written later.
+    float2* acc01;
+    float2* acc23;
     uint64_t* codes;     // Wo*Ho packed output codes + hole bit
     uint8_t* holes;      // Wo*Ho hole mask (1 = no view covers the pixel)
     uint64_t* scan[4];   // Wo*Ho inpainting scratch each
     uint64_t* inpaint_seg;  // column-group and warp-segment minima of the inpainting pre-passes
-    int* tile_order;        // output tiles, most bin entries first (raster launch order)
     float4* pcolor;      // Precision != 1: blended colour per raster pixel
     int32_t* psrc;       // Precision != 1: inpainting source of every hole
 };

@@ -57,24 +57,19 @@ RasterDims raster_dims(const rvsb_camera& virt, const rvsb_synth_params& p) {
     return {w, h, true};
 }
 
-int nblocks_x(int w) { return (w - 1 + BLOCK_W - 1) / BLOCK_W; }
-int nblocks_y(int h) { return (h - 1 + BLOCK_H - 1) / BLOCK_H; }
-
 namespace {
 
 struct SlotNeeds {
-    size_t vert, bbox, out, bins, list;
+    size_t vert, out, large;
 };
 
 SlotNeeds needs_of(const rvsb_scene* sc, int wo, int ho) {
     SlotNeeds n{};
-    for (const auto& c : sc->cams) {
-        n.vert += (size_t)c.width * c.height;
-        n.bbox += (size_t)nblocks_x(c.width) * nblocks_y(c.height);
-    }
+    for (const auto& c : sc->cams) n.vert += (size_t)c.width * c.height;
     n.out = (size_t)wo * ho;
-    n.bins = (size_t)((wo + MIN_TILE_W - 1) / MIN_TILE_W) * ((ho + MIN_TILE_H - 1) / MIN_TILE_H) * sc->cams.size();
-    n.list = std::min<size_t>(INT32_MAX / 2, std::max<size_t>(1 << 16, n.bbox * 8 + n.bins));
+    // About 1% of the triangles of an unmagnified view are large; when they
+    // do not fit, large_kernel goes over the whole mesh.
+    n.large = std::min<size_t>(INT32_MAX / 2, std::max<size_t>(1 << 14, n.vert / 11));
     return n;
 }
 
@@ -82,11 +77,8 @@ SlotNeeds needs_of(const rvsb_scene* sc, int wo, int ho) {
 
 size_t SlotWorkspace::bytes_for(const rvsb_scene* sc, int wo, int ho, bool rescale) {
     const SlotNeeds n = needs_of(sc, wo, ho);
-    return sizeof(DevStatus) + n.vert * sizeof(float4) + n.bbox * sizeof(int4) + 3 * n.bins * sizeof(int) +
-           n.list * sizeof(int) + n.out * (sizeof(uint64_t) * 5 + 1) +
-           inpaint_seg_words(wo) * sizeof(uint64_t) +
-           n.bins / std::max<size_t>(1, sc->cams.size()) * sizeof(int) +
-           (rescale ? n.out * (sizeof(float4) + 2 * sizeof(int32_t)) : 0);
+    return sizeof(DevStatus) + n.vert * sizeof(float4) + n.large * sizeof(uint4) + n.out * (sizeof(uint64_t) * 5 + 1) +
+           inpaint_seg_words(wo) * sizeof(uint64_t) + (rescale ? n.out * (sizeof(float4) + 2 * sizeof(int32_t)) : 0);
 }
 
 void SlotWorkspace::ensure_rescale(rvsb_context* ctx, int wo, int ho) {
@@ -105,24 +97,9 @@ void SlotWorkspace::ensure(rvsb_context* ctx, const rvsb_scene* sc, int wo, int 
         vert.alloc(ctx, n.vert * sizeof(float4));
         cap_vert = n.vert;
     }
-    if (n.bbox > cap_bbox) {
-        bbox.alloc(ctx, n.bbox * sizeof(int4));
-        cap_bbox = n.bbox;
-    }
-    if (n.bins > cap_bins) {
-        counts.alloc(ctx, n.bins * sizeof(int));
-        offsets.alloc(ctx, n.bins * sizeof(int));
-        cursor.alloc(ctx, n.bins * sizeof(int));
-        cap_bins = n.bins;
-    }
-    if (n.list > cap_list) {
-        list.alloc(ctx, n.list * sizeof(int));
-        cap_list = n.list;
-    }
-    const size_t tiles = (size_t)((wo + MIN_TILE_W - 1) / MIN_TILE_W) * ((ho + MIN_TILE_H - 1) / MIN_TILE_H);
-    if (tiles > cap_tiles) {
-        tile_order.alloc(ctx, tiles * sizeof(int));
-        cap_tiles = tiles;
+    if (n.large > cap_large) {
+        large.alloc(ctx, n.large * sizeof(uint4));
+        cap_large = n.large;
     }
     const size_t seg_words = inpaint_seg_words(wo);
     if (seg_words > cap_seg_words) {
@@ -132,7 +109,7 @@ void SlotWorkspace::ensure(rvsb_context* ctx, const rvsb_scene* sc, int wo, int 
     if (n.out > cap_out) {
         codes.alloc(ctx, n.out * sizeof(uint64_t));
         holes.alloc(ctx, n.out);
-        for (auto& s : scan) s.alloc(ctx, n.out * sizeof(uint64_t));
+        scan.alloc(ctx, 4 * n.out * sizeof(uint64_t));
         cap_out = n.out;
     }
 }
@@ -159,7 +136,6 @@ void SlotWorkspace::ensure_ms(rvsb_context* ctx, int n_views, int wo, int ho) {
 
 BatchCore::BatchCore(rvsb_context* ctx, int slots) : ctx_(ctx), slots_(slots) {
     if (slots <= 0) throw ArgError("a batch needs at least one slot");
-    prepare_kernels();
     for (int k = 0; k < slots; ++k) ws_.push_back(std::make_unique<SlotWorkspace>());
     tables_.alloc(ctx, sizeof(SlotTable) * (size_t)slots);
     for (int b = 0; b < 2; ++b) {
@@ -206,22 +182,16 @@ int BatchCore::stage_times(float* ms, int max_stages) const {
     return n;
 }
 
-namespace {
-int log2i(int v) {
-    int l = 0;
-    while ((1 << l) < v) ++l;
-    return l;
-}
-}  // namespace
-
-void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, int variant) {
+void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape& sh) {
     std::memset(&T, 0, sizeof(T));
     const rvsb_scene* sc = r.scene;
     SlotWorkspace& ws = *ws_[k];
     const rvsb_camera& virt = r.virt;
     const rvsb_synth_params& p = r.params;
     const int n = (int)sc->cams.size();
-    size_t voff = 0, boff = 0;
+    const RasterDims rd = raster_dims(virt, p);
+    const size_t npix = (size_t)rd.w * rd.h;
+    size_t voff = 0;
     for (int v = 0; v < n; ++v) {
         const rvsb_camera& c = sc->cams[v];
         DevView& V = T.v[v];
@@ -256,16 +226,12 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, int variant) {
         V.color = sc->color[v]->as<uint64_t>();
         V.depth_lut = sc->depth_lut[v]->as<float4>();
         V.vert = ws.vert.as<float4>() + voff;
-        V.bbox = ws.bbox.as<int4>() + boff;
+        V.z = ws.scan.as<unsigned long long>() + (size_t)(v % sh.vg) * npix;
         V.tri_shift = 2;
         while ((1 << (V.tri_shift - 2)) < c.width - 1) ++V.tri_shift;
-        V.nbx = nblocks_x(c.width);
-        V.nby = nblocks_y(c.height);
         voff += (size_t)c.width * c.height;
-        boff += (size_t)V.nbx * V.nby;
     }
     DevTarget& D = T.t;
-    const RasterDims rd = raster_dims(virt, p);
     D.wo = rd.w;
     D.ho = rd.h;
     D.out_w = virt.width;
@@ -333,25 +299,17 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, int variant) {
         M.low_int = exp_int(p.low_freq_factor);
         M.high_int = exp_int(p.high_freq_factor);
     }
-    const RasterVariant& rv = kRasterVariants[variant];
-    D.tile_wl = log2i(rv.tw);
-    D.tile_hl = log2i(rv.th);
-    D.ntx = (rd.w + rv.tw - 1) / rv.tw;
-    D.nty = (rd.h + rv.th - 1) / rv.th;
     D.n_views = n;
-    D.bin_capacity = (int)ws.cap_list;
     SlotBuffers& B = T.b;
     B.status = ws.status.as<DevStatus>();
-    B.counts = ws.counts.as<int>();
-    B.offsets = ws.offsets.as<int>();
-    B.cursor = ws.cursor.as<int>();
-    B.list = ws.list.as<int>();
-    B.capacity = (int)ws.cap_list;
+    B.large = ws.large.as<uint4>();
+    B.large_capacity = (int)ws.cap_large;
     B.codes = ws.codes.as<uint64_t>();
     B.holes = ws.holes.as<uint8_t>();
-    for (int s = 0; s < 4; ++s) B.scan[s] = ws.scan[s].as<uint64_t>();
+    for (int s = 0; s < 4; ++s) B.scan[s] = ws.scan.as<uint64_t>() + (size_t)s * npix;
+    B.acc01 = reinterpret_cast<float2*>(B.scan[3]);
+    B.acc23 = reinterpret_cast<float2*>(B.codes);
     B.inpaint_seg = ws.inpaint_seg.as<uint64_t>();
-    B.tile_order = ws.tile_order.as<int>();
     if (rd.rescale) {
         B.pcolor = ws.pcolor.as<float4>();
         B.psrc = r.dbg.inpaint_source ? r.dbg.inpaint_source : ws.psrc.as<int32_t>();
@@ -379,33 +337,30 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, int variant) {
 }
 
 BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) const {
-    const RasterVariant& rv = kRasterVariants[variant];
     BatchShape sh;
     sh.slots = n;
     sh.variant = variant;
     for (int k = 0; k < n; ++k) {
-        if (reqs[k].aux) sh.aux = 1;
-        if (reqs[k].params.blending_method == RVSB_BLEND_MULTISPECTRAL) sh.ms = 1;
-        if (reqs[k].params.precision != 1.f) sh.rescale = 1;
-    }
-    for (int k = 0; k < n; ++k) {
         const SlotRequest& r = reqs[k];
-        const int nv = (int)r.scene->cams.size();
-        sh.max_views = std::max(sh.max_views, nv);
+        if (r.aux) sh.aux = 1;
+        if (r.params.blending_method == RVSB_BLEND_MULTISPECTRAL) sh.ms = 1;
+        if (r.params.precision != 1.f) sh.rescale = 1;
+        if (r.aux || r.dbg.any() || r.params.blending_method == RVSB_BLEND_MULTISPECTRAL) sh.extras = 1;
+        sh.max_views = std::max(sh.max_views, (int)r.scene->cams.size());
         for (const auto& c : r.scene->cams) {
             sh.max_w = std::max(sh.max_w, c.width);
             sh.max_h = std::max(sh.max_h, c.height);
-            sh.max_blocks = std::max(sh.max_blocks, nblocks_x(c.width) * nblocks_y(c.height));
         }
         const RasterDims rd = raster_dims(r.virt, r.params);
-        const int ntiles = ((rd.w + rv.tw - 1) / rv.tw) * ((rd.h + rv.th - 1) / rv.th);
         sh.max_wo = std::max(sh.max_wo, rd.w);
         sh.max_ho = std::max(sh.max_ho, rd.h);
         sh.max_out_w = std::max(sh.max_out_w, r.virt.width);
         sh.max_out_h = std::max(sh.max_out_h, r.virt.height);
-        sh.max_tiles = std::max(sh.max_tiles, ntiles);
-        sh.max_bins = std::max(sh.max_bins, ntiles * nv);
     }
+    // The four words per pixel that the inpainting scans use later hold the
+    // z-buffers of up to four views, or, for more views, of three at a time
+    // and half of the running blend (its other half takes the codes').
+    sh.vg = sh.max_views <= 4 ? 4 : 3;
     return sh;
 }
 
@@ -414,7 +369,7 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
     if (n == 1 && !use_graphs_) {
         // A single synthesis: the table travels as a kernel parameter.
         TableParam tp;
-        fill(tp.t, 0, reqs[0], variant);
+        fill(tp.t, 0, reqs[0], sh);
         const int launches = launch_batch(tp, sh, s, profiling_ ? events_ : nullptr);
         if (launches < 0) check(cudaGetLastError(), "kernel launch");
         return launches;
@@ -422,16 +377,15 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
     // The staging buffer is reused every other call: its previous copy must
     // have been consumed.
     check(cudaEventSynchronize(copied_[cur_]), "wait for table staging");
-    for (int k = 0; k < n; ++k) fill(staging_[cur_][k], k, reqs[k], variant);
+    for (int k = 0; k < n; ++k) fill(staging_[cur_][k], k, reqs[k], sh);
     check(cudaMemcpyAsync(tables_.ptr, staging_[cur_], sizeof(SlotTable) * (size_t)n, cudaMemcpyHostToDevice, s),
           "upload slot tables");
     check(cudaEventRecord(copied_[cur_], s), "record table upload");
     cur_ ^= 1;
     const TablePtr tabs{tables_.as<SlotTable>()};
     if (use_graphs_ && !profiling_) {
-        const std::vector<int> key = {sh.slots,  sh.variant, sh.max_views, sh.max_w,    sh.max_h,
-                                      sh.max_blocks, sh.max_wo, sh.max_ho, sh.max_tiles, sh.max_bins, sh.aux, sh.ms,
-                                      sh.rescale, sh.max_out_w, sh.max_out_h};
+        const std::vector<int> key = {sh.slots, sh.variant, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
+                                      sh.max_ho, sh.aux, sh.ms, sh.extras, sh.rescale, sh.max_out_w, sh.max_out_h};
         auto it = graphs_.find(key);
         if (it == graphs_.end()) {
             cudaGraph_t g = nullptr;
@@ -467,47 +421,12 @@ float pixels_per_radian(const rvsb_camera& c) {
     return c.focal[0];
 }
 
-// Raster variant of a run that is neither pinned nor tuned.  An input pixel
-// spacing seen m times magnified in the raster gives triangles whose
-// candidate boxes hold about (m + 1)^2 pixels, so past m of about 1 most
-// leave the small path (at most 4 candidates) and the medium path of variant
-// 7 rasterises them faster: 960x540 inputs into a 1920x1080 output (m = 2)
-// 0.359 -> 0.285 ms, 4096x2048 equirectangular inputs into 1920x1080
-// (m = 1.47) 1.03 -> 0.62 ms; at m <= 1 it is 2 to 26% slower.  An
-// equirectangular output stretches its rows by 1 / cos(latitude), sqrt(2) at
-// the median row, which its m includes (equirectangular to equirectangular
-// at m = 1: 4.30 -> 3.25 ms).  The largest m of the batch decides.
-// At m <= 1.1 variant 4 (64x32 tiles, all four views in one z-buffer
-// group, 1024-thread CTAs, one per SM) runs: a binning block lands in 1.35
-// of its tiles instead of 1.53 of 32x32, the bins are half as many, and a
-// tile's 32 warps finish it in about half the time of 16, which keeps the
-// last wave short.  Against variant 0 (ms per view, median of 36 calls):
-// 4 x 1920x1080 into 1920x1080 0.648 -> 0.621, into 960x540 0.459 -> 0.453,
-// into an equirectangular 4096x2048 1.027 -> 0.943; 2 x 960x540 into
-// 960x540 0.153 -> 0.150.  A perspective output minified to m <= 0.6 has
-// many small triangles per tile, and the 32x32 tiles of variant 2 (also
-// 1024-thread CTAs) rasterise it faster: 4 x 1920x1080 into 960x540 (m =
-// 0.5) 0.450 -> 0.406 ms, into 640x360 (m = 0.33) 0.521 -> 0.440 ms; at m =
-// 0.67 variant 4 is ahead again (0.452 against 0.466).  A batch of many
-// slots has tiles enough that the last wave does not matter, and there two
-// 512-thread CTAs per SM, one working while the other waits at a barrier,
-// do better: variant 1 (64x32 tiles of two views) runs 16 poses of the
-// 1080p scene at 1806 views/s and the 64-target mixed batch at 771,
-// against 755 for variant 4.
+// Raster variant of a run that is neither pinned nor tuned.
 constexpr int kMagnifiedVariant = 7;
 constexpr int kDefaultVariant = 4;
 constexpr int kMinifiedVariant = 2;
 constexpr int kBatchVariant = 1;
 constexpr int kBatchVariantMinSlots = 8;
-static_assert(kRasterVariants[kMagnifiedVariant].med > kRasterVariants[kMagnifiedVariant].small,
-              "the magnified default has the medium-triangle path");
-static_assert(kRasterVariants[kDefaultVariant].tw == 64 && kRasterVariants[kDefaultVariant].vg == 4 &&
-                  kRasterVariants[kDefaultVariant].threads == 1024,
-              "the default holds 64x32 tiles of four views in 1024-thread CTAs");
-static_assert(kRasterVariants[kMinifiedVariant].tw == 32 && kRasterVariants[kMinifiedVariant].threads == 1024,
-              "the minified default holds 32x32 tiles in 1024-thread CTAs");
-static_assert(kRasterVariants[kBatchVariant].threads == 512 && kRasterVariants[kBatchVariant].med == 0,
-              "the batch default runs two CTAs per SM");
 
 int default_variant(const SlotRequest* reqs, int n) {
     float m = 0.f;

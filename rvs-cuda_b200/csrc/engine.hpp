@@ -75,21 +75,22 @@ struct DevMem {
 };
 
 // Buffers of one synthesis slot, grown on demand to the largest request
-// seen: the warped vertices and block boxes of every input view, the bins,
-// and the output-sized codes, hole mask and inpainting scratch.
+// seen: the warped vertices of every input view, the list of large
+// triangles, and the output-sized z-buffers, codes, hole mask and inpainting
+// scratch.
 struct SlotWorkspace {
-    DevMem status, counts, offsets, cursor, list, codes, holes, scan[4], vert, bbox;
+    DevMem status, codes, holes, vert;
+    DevMem scan;                  // 4 words per output pixel: the z-buffers, then the inpainting scans
+    DevMem large;                 // list of large triangles
     DevMem aux_depth, aux_valid;  // blended depth / validity (auxiliary outputs only)
     DevMem inpaint_seg;           // column-group minima of the inpainting passes
-    DevMem tile_order;            // raster launch order of the output tiles
-    size_t cap_tiles = 0;
     DevMem ms_view, ms_hsum, ms_hcnt, ms_blur;  // multispectral blending only
     size_t cap_ms = 0;            // view-pixels the multispectral buffers hold
     void ensure_ms(rvsb_context* ctx, int n_views, int wo, int ho);
     DevMem pcolor, psrc;          // Precision != 1: raster-size colour and inpainting sources
     size_t cap_rescale = 0;
     void ensure_rescale(rvsb_context* ctx, int wo, int ho);
-    size_t cap_vert = 0, cap_bbox = 0, cap_out = 0, cap_bins = 0, cap_list = 0, cap_aux = 0, cap_seg_words = 0;
+    size_t cap_vert = 0, cap_out = 0, cap_large = 0, cap_aux = 0, cap_seg_words = 0;
     void ensure_aux(rvsb_context* ctx, int wo, int ho);
 
     // Bytes a slot needs for `scene` at raster size wo x ho (rescale: plus
@@ -109,10 +110,6 @@ struct RasterDims {
     bool rescale;
 };
 RasterDims raster_dims(const rvsb_camera& virt, const rvsb_synth_params& p);
-
-// Number of binning blocks of a view (BLOCK_W x BLOCK_H quads).
-int nblocks_x(int w);
-int nblocks_y(int h);
 
 // One synthesis request of a batch.
 struct SlotRequest {
@@ -156,7 +153,7 @@ public:
     int last_launches() const { return last_launches_; }
 
 private:
-    void fill(SlotTable& t, int k, const SlotRequest& r, int variant);
+    void fill(SlotTable& t, int k, const SlotRequest& r, const BatchShape& sh);
     BatchShape shape_of(const SlotRequest* reqs, int n, int variant) const;
     int launch_variant(const SlotRequest* reqs, int n, int variant, cudaStream_t s);
     int tune(const SlotRequest* reqs, int n, cudaStream_t s);

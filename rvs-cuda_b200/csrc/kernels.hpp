@@ -14,12 +14,11 @@ struct BatchShape {
     int variant = 0;         // raster variant (kRasterVariants)
     int aux = 0;             // some slot wants auxiliary outputs
     int ms = 0;              // some slot blends multispectrally
+    int extras = 0;          // some slot wants per-view, auxiliary or debug outputs of the resolve
     int max_views = 0;       // largest n_views
+    int vg = 4;              // views per z-buffer group
     int max_w = 0, max_h = 0;  // largest input view
-    int max_blocks = 0;      // largest nbx * nby of an input view
     int max_wo = 0, max_ho = 0;
-    int max_tiles = 0;       // largest ntx * nty
-    int max_bins = 0;        // largest ntx * nty * n_views
     int rescale = 0;         // some slot rasterises at Precision != 1
     int max_out_w = 0, max_out_h = 0;  // largest output (virtual camera) size
 };
@@ -69,32 +68,23 @@ constexpr int NUM_STAGES = 5;
 template <class Tabs>
 int launch_batch(const Tabs& tabs, const BatchShape& shape, cudaStream_t stream, cudaEvent_t* events = nullptr);
 
-// Raster variants the autotuner chooses from: tile width and height, views
-// per shared z-buffer group, the candidate count above which a triangle is
-// rasterised warp-cooperatively, the bin entries staged per round, and the
-// candidate count up to which those triangles are flattened across the warp
-// together (med <= small: each one alone, row span by row span).  Every
-// variant gives identical results.
+// Raster variants the autotuner chooses from: quad rows per warp of the mesh
+// kernel and the candidate pixels above which a triangle goes to the list of
+// large ones.  Every variant gives identical results.
 struct RasterVariant {
-    int tw, th, vg, small, ent, med, threads;
+    int rows, small;
 };
 constexpr int NUM_RASTER_VARIANTS = 8;
 constexpr RasterVariant kRasterVariants[NUM_RASTER_VARIANTS] = {
-    {32, 32, 4, 4, 1024, 0, 512},  {64, 32, 2, 4, 1024, 0, 512},   {32, 32, 4, 4, 1024, 0, 1024},
-    {32, 32, 4, 8, 1024, 0, 512},  {64, 32, 4, 4, 1024, 0, 1024},  {64, 32, 2, 4, 1024, 32, 1024},
-    {32, 32, 4, 2, 1024, 32, 512}, {64, 32, 2, 4, 1024, 32, 512},
+    {16, 4}, {16, 8}, {32, 4}, {32, 8}, {16, 8}, {8, 16}, {16, 64}, {16, 16},
 };
-// The bin arrays are sized for tiles of MIN_TILE_W x MIN_TILE_H.
-constexpr bool tiles_at_least_minimum() {
+constexpr bool rows_divide_tiles() {
     for (const RasterVariant& v : kRasterVariants)
-        if (v.tw < MIN_TILE_W || v.th < MIN_TILE_H) return false;
+        if (WARP_TILE % v.rows != 0) return false;
     return true;
 }
-static_assert(tiles_at_least_minimum(), "a raster variant's tiles are smaller than the bins are sized for");
+static_assert(rows_divide_tiles(), "a warp's quad rows must lie in one row of culling tiles");
 
-// One-time kernel attributes of the current device (the raster kernel's
-// dynamic shared memory); call before launching or capturing a batch.
-void prepare_kernels();
 // Shared memory of the multispectral row sums for outputs up to max_wo wide.
 void prepare_ms_kernels(int max_wo);
 

@@ -1,0 +1,599 @@
+// Mesh stage: warps every input pixel and rasterises the triangles of its
+// quads straight away into the views' z-buffers.
+//
+// A z-buffer holds one 64-bit key per output pixel of a view,
+//   (bits of depth^3 / quality) << 32 | triangle scan index,
+// and a fragment is one 64-bit atomicMin on it, so the winner does not depend
+// on scheduling.  The buffers live in global memory: the views one launch
+// works on at a time take tens of megabytes, which the 126 MB L2 holds, and
+// a warp's fragments lie in a few rows of neighbouring pixels.  Against
+// z-buffers in shared memory per output tile this needs no binning of the
+// triangles into tiles (a count, a scan and a fill pass), sets every triangle
+// up once instead of once per tile its 8x4-quad block touches (1.35 times on
+// the 4 x 1920x1080 view), holds nothing at block barriers, and takes the
+// vertices from registers instead of reading the warped mesh back.  Measured
+// for the whole call (shared-memory tiles -> this): 4 x 1920x1080 ->
+// 1920x1080 598 -> 457 us, -> 960x540 415 -> 267 us, 4 x ERP 4096x2048 -> ERP
+// 3062 -> 2010 us, 2 x 960x540 -> 960x540 132 -> 118 us.
+//
+// mesh_kernel: one warp takes a strip of 32 vertex columns (31 quads) and
+// `rows` rows of quads, a lane one column: it warps the row below, gets the
+// right neighbour's vertices by shuffles, and rasterises the two triangles of
+// its quad.  Triangles of up to SMALL candidate pixels are tested by their
+// lane; larger ones (stretched over depth discontinuities) go to the slot's
+// list and large_kernel rasterises them, one warp per entry, lanes over the
+// pixels of their row spans.
+#include <algorithm>
+
+#include "device_common.cuh"
+#include "kernels.hpp"
+
+namespace rvsb {
+namespace {
+
+using namespace dev;
+
+constexpr int MESH_WARPS = 4;
+constexpr int STRIP = 31;              // quads (columns) per warp
+constexpr int QUEUE = 64;              // large triangles a warp holds before they go to the list
+constexpr int LARGE_THREADS = 128;
+// Most candidate pixels of one list entry: a larger box is entered as
+// several bands of rows, so that one triangle over much of the output does
+// not keep a single warp busy after all others are done.
+constexpr int kEntryPixels = 4096;
+
+// Adding 1.5 * 2^23 rounds a float to the nearest integer and leaves it in
+// the low mantissa bits, and for any float the result's bits, compared as
+// int, order as the value does; so pixel coordinates stay in this biased form
+// through the clamping and the loop (no conversions).
+constexpr float kBias = 12582912.f;
+constexpr int kBiasBits = 0x4B400000;
+
+// Reciprocal of a normal number, the same result as rcp_approx.
+__device__ __forceinline__ float rcp_normal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The view's fields the warp uses per vertex (tab.v[view] is indexed by the
+// grid, so each use would otherwise be a load).
+struct RegView {
+    int w, h, proj;
+    float p0, p1;
+    float R[9], t[3];
+    const uint16_t* pd;
+    const float4* depth_lut;
+    const float* erp_row;
+    const float* erp_col;
+    __device__ explicit RegView(const DevView& G) {
+        w = G.w; h = G.h; proj = G.proj; p0 = G.p0; p1 = G.p1;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) R[k] = G.R[k];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) t[k] = G.t[k];
+        pd = G.pd; depth_lut = G.depth_lut; erp_row = G.erp_row; erp_col = G.erp_col;
+    }
+};
+
+// Whether vertex tile (tx, ty) of an ERP input view lies, with
+// its one-pixel ring, wholly beyond one of the output's side planes.  A
+// vertex is x = z * d (d within the tile's cone, z within its depth range),
+// seen by the virtual camera as y = R x + t; beyond plane a when a . y > 0,
+// i.e. z * (b . d) + c > 0 with b = R^T a, c = a . t.  Over the cone
+// b . d >= b . dc - |b| rho; the smallest value over z is at the near or far
+// end of the range.  A relative margin absorbs the float rounding of the
+// vertices, and the planes sit one pixel outside the image.
+__device__ __forceinline__ bool tile_culled(const DevView& V, const DevTarget& T, int tx, int ty) {
+    const int ntx = (V.w + WARP_TILE - 1) / WARP_TILE;
+    const size_t k = (size_t)ty * ntx + tx;
+    const float4 cone = V.erp_cone[k];
+    const float2 zr = V.tile_depth[k];
+    if (!(zr.x > 0.f && zr.x <= zr.y)) return false;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const float* a = T.cull_plane[p];
+        float b[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) b[j] = a[0] * V.R[j] + a[1] * V.R[3 + j] + a[2] * V.R[6 + j];
+        const float c = a[0] * V.t[0] + a[1] * V.t[1] + a[2] * V.t[2];
+        const float nb = sqrtf(b[0] * b[0] + b[1] * b[1] + b[2] * b[2]);
+        const float m = b[0] * cone.x + b[1] * cone.y + b[2] * cone.z - nb * cone.w;
+        const float z = m >= 0.f ? zr.x : zr.y;
+        const float L = z * m + c;
+        if (L > 1e-3f * (fabsf(c) + z * nb) && isfinite(L)) return true;
+    }
+    return false;
+}
+
+// What the rasterisation of one view's triangles needs beside the triangle.
+struct MeshTarget {
+    unsigned long long* z;
+    int wo;
+    uint32_t origin;         // biased index (y * wo + x) of pixel (0, 0)
+    int xmin, xmax, ymin, ymax;  // pixel range, biased
+    float precision;
+};
+
+__device__ __forceinline__ float sq2(float dx, float dy) {
+    return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+}
+
+// Key word of a fragment (see key_invq): bits of d^3 / quality.
+__device__ __forceinline__ float small_invq(float m, float precision) {
+    float stretch = __fsqrt_rn(m);
+    if (precision != 1.f) stretch = __fdiv_rn(stretch, precision);
+    return rcp_normal(fminf(10000.f, fmaxf(1.f, __fsub_rn(10000.f, __fmul_rn(1000.f, stretch)))));
+}
+
+// One triangle of a lane's quad (edge coefficients as in tri_coef; mn and mx:
+// its bounding box; m2: its longest edge squared).  Returns its candidate
+// box through `box` with `large` set when it belongs in the list.
+//
+// Candidate range: a covered pixel's centre lies within the bounding box
+// grown by the tolerance tri_range (device_common.cuh) derives, and
+// round(mn - delta) .. round(mx + delta) - 1 holds every such pixel and, for
+// delta < 0.5, nothing outside the CPU's box [floor(min), ceil(max)].
+// Triangles wider than 4e4 pixels (there the CPU's box and the tolerance
+// need care) and those with a nearly zero determinant are left to the list.
+//
+// Coverage: the test of test_pixel (below) with its error bound
+// taken at M = 1.  The bound 24u * M on each coordinate is derived there from
+// one of 21u * M, so for M < 24/21 the constant 24u still holds; and since
+// the three coordinates add up to 1, M >= 24/21 puts the smallest below
+// -(M - 1) / 2 < -0.07, far outside.
+template <int SMALL>
+__device__ __forceinline__ bool raster_small(const MeshTarget& o, bool active, float b1c1, float c0b0, float c1a1,
+                                             float a0c0, float cx, float cy, float za, float zb, float zc, float mnx,
+                                             float mxx, float mny, float mxy, float m2, uint32_t tri, int4& box,
+                                             bool& wide) {
+    const float u = 5.9604645e-8f, eps = 1e-6f;
+    const float den = __fsub_rn(__fmul_rn(b1c1, a0c0), __fmul_rn(c0b0, c1a1));
+    const float L = fmaxf(__fsub_rn(mxx, mnx), __fsub_rn(mxy, mny));
+    wide = !(L < 4.0e4f);
+    const float delta = wide ? 2.f : __fmaf_rn(1e-5f, L, 4e-3f);
+    box.x = max(o.xmin, __float_as_int(__fadd_rn(__fsub_rn(mnx, delta), kBias)));
+    box.y = max(o.ymin, __float_as_int(__fadd_rn(__fsub_rn(mny, delta), kBias)));
+    box.z = min(o.xmax, __float_as_int(__fadd_rn(__fadd_rn(mxx, delta), kBias)) - 1);
+    box.w = min(o.ymax, __float_as_int(__fadd_rn(__fadd_rn(mxy, delta), kBias)) - 1);
+    if (!(active && den > 0.f && box.x <= box.z && box.y <= box.w)) return false;
+    const int count = (box.z - box.x + 1) * (box.w - box.y + 1);
+    if (wide || count > SMALL || !(den >= 1e-30f)) return true;
+    const float rinv = rcp_normal(den);
+    const float invq = small_invq(m2, o.precision);
+    int xb = box.x, yb = box.y;
+    for (int k = count; k > 0; --k) {
+        const float tx = __fsub_rn(__fadd_rn(__fsub_rn(__int_as_float(xb), kBias), 0.5f), cx);
+        const float ty = __fsub_rn(__fadd_rn(__fsub_rn(__int_as_float(yb), kBias), 0.5f), cy);
+        const float n1 = __fadd_rn(__fmul_rn(b1c1, tx), __fmul_rn(c0b0, ty));
+        const float n2 = __fadd_rn(__fmul_rn(c1a1, tx), __fmul_rn(a0c0, ty));
+        float l1 = __fmul_rn(n1, rinv), l2 = __fmul_rn(n2, rinv);
+        float l3 = __fsub_rn(__fsub_rn(1.f, l1), l2);
+        const float mn = fminf(fminf(l1, l2), l3);
+        bool in = mn >= -eps + 24.f * u;
+        if (!in && mn >= -eps - 24.f * u) {
+            l1 = __fdiv_rn(n1, den);
+            l2 = __fdiv_rn(n2, den);
+            l3 = __fsub_rn(__fsub_rn(1.f, l1), l2);
+            in = covered(l1, l2, l3);
+        }
+        if (in) {
+            const float d = interp(za, zb, zc, l1, l2, l3);
+            if (!isnan(d)) {
+                uint32_t hi = 0u;
+                if (d > 0.f) hi = __float_as_uint(__fmul_rn(__fmul_rn(__fmul_rn(d, d), d), invq));
+                atomicMin(o.z + ((uint32_t)yb * (uint32_t)o.wo + (uint32_t)xb - o.origin), ((unsigned long long)hi << 32) | tri);
+            }
+        }
+        if (++xb > box.z) {
+            xb = box.x;
+            ++yb;
+        }
+    }
+    return false;
+}
+
+// A warp's large triangles on their way to the slot's list: at most 31 wait
+// in the warp's queue in shared memory; full groups of 32 go out together
+// (one atomic on the list's length, coalesced 16-byte stores).
+struct LargeQueue {
+    uint4* q;       // QUEUE entries of this warp
+    int n;
+    __device__ void flush(const SlotBuffers& B, int lane, int count) {
+        __syncwarp();
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&B.status->n_large, count);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (lane < count) {
+            // Past the capacity the entry is dropped; large_kernel sees the
+            // length and goes over the whole mesh instead.
+            if (base + lane < B.large_capacity) B.large[base + lane] = q[lane];
+        }
+        __syncwarp();
+        const uint4 rest = q[32 + lane];
+        __syncwarp();
+        q[lane] = rest;
+        n -= count;
+        __syncwarp();
+    }
+    // Entered by the whole warp; `push` lanes have a triangle with box `b`
+    // (biased).  Boxes of more than kEntryPixels pixels become bands of rows.
+    __device__ void push(const SlotBuffers& B, int lane, bool push, uint32_t tri, int view, bool general, int4 b) {
+        const int w = b.z - b.x + 1;
+        const int band = general ? 1 << 20 : max(1, kEntryPixels / max(1, w));
+        int y = b.y;
+        unsigned m;
+        while ((m = __ballot_sync(0xffffffffu, push))) {
+            if (push) {
+                const int ye = min(b.w, y + band - 1);
+                q[n + __popc(m & ((1u << lane) - 1u))] =
+                    make_uint4(tri, (uint32_t)view | (general ? 256u : 0u),
+                               (uint32_t)(b.x - kBiasBits) | ((uint32_t)(b.z - kBiasBits) << 16),
+                               (uint32_t)(y - kBiasBits) | ((uint32_t)(ye - kBiasBits) << 16));
+                y = ye + 1;
+                push = y <= b.w;
+            }
+            n += __popc(m);
+            if (n >= 32) flush(B, lane, 32);
+        }
+    }
+};
+
+// Grid (ceil(strips / MESH_WARPS), ceil(max quad rows / rows), slots * gv):
+// views g0 .. g0 + gv - 1 of every slot.  ERP outputs wrapping horizontally
+// have one more strip, whose lanes take the seam triangles of one row each.
+template <int SMALL, class Tabs>
+__global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_constant__ Tabs tabs, int g0, int gv,
+                                                                   int rows) {
+    __shared__ uint4 s_queue[MESH_WARPS][QUEUE];
+    grid_dep_wait();
+    const SlotTable& tab = tabs.at(blockIdx.z / gv);
+    const int view = g0 + blockIdx.z % gv;
+    const DevTarget& T = tab.t;
+    if (view >= T.n_views) return;
+    const DevView& G = tab.v[view];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int strip = blockIdx.x * MESH_WARPS + warp, i0 = blockIdx.y * rows;
+    const int nstrips = (G.w - 1 + STRIP - 1) / STRIP;
+    const bool seam = T.wrap != 0 && strip == nstrips;
+    if (i0 >= G.h - 1 || (strip >= nstrips && !seam)) return;
+    const int i1 = min(i0 + rows, G.h - 1);  // last vertex row of the warp's quads
+    const int j = strip * STRIP + lane;
+    bool keep_all = false;
+    if (T.cull && G.erp_cone) {
+        // Quad rows i0 .. i1 - 1 lie in one row of vertex tiles (rows divides
+        // WARP_TILE) and the strip's quads in at most two tiles of it; every
+        // quad's corners lie in its tile grown by one pixel.
+        const int t0 = strip * STRIP / WARP_TILE, t1 = min(strip * STRIP + STRIP - 1, G.w - 2) / WARP_TILE;
+        const bool live = t0 + lane <= t1 && !tile_culled(G, T, t0 + lane, i0 / WARP_TILE);
+        if (!__any_sync(0xffffffffu, live)) return;
+        // The strips right of and below this one may be skipped: the last
+        // column and row are stored here as well.
+        keep_all = true;
+    }
+    MeshTarget o;
+    o.wo = T.wo;
+    o.xmin = o.ymin = kBiasBits;
+    o.xmax = kBiasBits + T.wo - 1;
+    o.ymax = kBiasBits + T.ho - 1;
+    o.z = G.z;
+    o.origin = (uint32_t)kBiasBits * (uint32_t)T.wo + (uint32_t)kBiasBits;
+    o.precision = T.precision;
+    const RegView V(G);
+    float4* vert = G.vert;
+    const int shift = G.tri_shift;
+    LargeQueue queue{s_queue[warp], 0};
+    if (!seam) {
+        const bool in_col = j < V.w;
+        const bool store = in_col && (lane < STRIP || j == V.w - 1 || keep_all);
+        const int jc = min(j, V.w - 1);
+        float4 L = depth_entry(V, i0, jc);
+        uint16_t raw = __ldg(V.pd + (size_t)min(i0 + 2, i1) * V.w + jc);
+        float4 Ln = depth_entry(V, i0 + 1, jc);
+        float4 a = warp_vertex(V, T, i0, jc, L);
+        if (store) vert[(size_t)i0 * V.w + j] = a;
+        // Emission test (transform.cpp:161-167) per vertex, as masks of the row.
+        unsigned ok_a = __ballot_sync(0xffffffffu, a.z > 0.f && a.x > 0.f);
+        const unsigned quads = __ballot_sync(0xffffffffu, lane < STRIP && j + 1 < V.w);
+        float bx = __shfl_down_sync(0xffffffffu, a.x, 1), by = __shfl_down_sync(0xffffffffu, a.y, 1),
+              bz = __shfl_down_sync(0xffffffffu, a.z, 1);
+        for (int i = i0; i < i1; ++i) {
+            L = Ln;
+            Ln = __ldg(V.depth_lut + raw);
+            raw = __ldg(V.pd + (size_t)min(i + 3, i1) * V.w + jc);
+            const float4 c = warp_vertex(V, T, i + 1, jc, L);
+            if (store && (i + 1 < i1 || i1 == V.h - 1 || keep_all)) vert[(size_t)(i + 1) * V.w + j] = c;
+            const unsigned ok_c = __ballot_sync(0xffffffffu, c.z > 0.f && c.x > 0.f);
+            const float dx = __shfl_down_sync(0xffffffffu, c.x, 1), dy = __shfl_down_sync(0xffffffffu, c.y, 1),
+                        dz = __shfl_down_sync(0xffffffffu, c.z, 1);
+            const unsigned cond = (ok_a >> 1) & ok_c & quads;
+            if (cond) {
+                const uint32_t tri = (((uint32_t)i << (shift - 2)) | (uint32_t)j) * 4u;
+                // The diagonal b - c belongs to both triangles: its
+                // differences, squared length and box serve both (negated
+                // exactly for the second).
+                const float ey = __fsub_rn(by, c.y), ex = __fsub_rn(c.x, bx);
+                const float md = sq2(ex, ey);
+                const float nx = fminf(bx, c.x), xx = fmaxf(bx, c.x), ny = fminf(by, c.y), xy = fmaxf(by, c.y);
+                int4 box;
+                bool wide, big;
+                {
+                    const float a0c0 = __fsub_rn(a.x, c.x), c1a1 = __fsub_rn(c.y, a.y);
+                    const float m2 = fmaxf(md, fmaxf(sq2(a0c0, c1a1), sq2(__fsub_rn(a.x, bx), __fsub_rn(a.y, by))));
+                    big = raster_small<SMALL>(o, (cond & ok_a) >> lane & 1u, ey, ex, c1a1, a0c0, c.x, c.y, a.z, bz,
+                                              c.z, fminf(nx, a.x), fmaxf(xx, a.x), fminf(ny, a.y), fmaxf(xy, a.y), m2,
+                                              tri, box, wide);
+                    if (__any_sync(0xffffffffu, big)) queue.push(tab.b, lane, big, tri, view, wide, box);
+                }
+                {
+                    const float a0c0 = __fsub_rn(dx, bx), c1a1 = __fsub_rn(by, dy);
+                    const float m2 = fmaxf(md, fmaxf(sq2(a0c0, c1a1), sq2(__fsub_rn(dx, c.x), __fsub_rn(dy, c.y))));
+                    big = raster_small<SMALL>(o, (cond & (ok_c >> 1)) >> lane & 1u, -ey, -ex, c1a1, a0c0, bx, by, dz,
+                                              c.z, bz, fminf(nx, dx), fmaxf(xx, dx), fminf(ny, dy), fmaxf(xy, dy), m2,
+                                              tri + 1u, box, wide);
+                    if (__any_sync(0xffffffffu, big)) queue.push(tab.b, lane, big, tri + 1u, view, wide, box);
+                }
+            }
+            a = c;
+            bx = dx;
+            by = dy;
+            bz = dz;
+            ok_a = ok_c;
+        }
+    } else {
+        // Seam triangles (transform.cpp:168-175), between columns W - 1 and 0
+        // of quad row i0 + lane: emitted where quad (i, 0)'s diagonal is.
+        const int i = min(i0 + lane, i1 - 1);
+        const float4 v00 = warp_vertex(V, T, i, 0), v01 = warp_vertex(V, T, i, 1), v10 = warp_vertex(V, T, i + 1, 0);
+        const float4 w0 = warp_vertex(V, T, i, V.w - 1), w1 = warp_vertex(V, T, i + 1, V.w - 1);
+        const bool active = i0 + lane < i1 && v01.z > 0.f && v10.z > 0.f && v01.x > 0.f && v10.x > 0.f;
+        const uint32_t tri = ((uint32_t)i << shift) | 2u;
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) {
+            const float4 A = t ? v10 : w0, B = t ? w1 : v00, C = t ? v00 : w1;
+            const float b1c1 = __fsub_rn(B.y, C.y), c0b0 = __fsub_rn(C.x, B.x), a0c0 = __fsub_rn(A.x, C.x),
+                        c1a1 = __fsub_rn(C.y, A.y);
+            const float m2 = fmaxf(sq2(c0b0, b1c1),
+                                   fmaxf(sq2(a0c0, c1a1), sq2(__fsub_rn(A.x, B.x), __fsub_rn(A.y, B.y))));
+            int4 box;
+            bool wide;
+            const bool big = raster_small<SMALL>(
+                o, active, b1c1, c0b0, c1a1, a0c0, C.x, C.y, A.z, B.z, C.z, fminf(fminf(A.x, B.x), C.x),
+                fmaxf(fmaxf(A.x, B.x), C.x), fminf(fminf(A.y, B.y), C.y), fmaxf(fmaxf(A.y, B.y), C.y), m2,
+                tri + (uint32_t)t, box, wide);
+            queue.push(tab.b, lane, big, tri + (uint32_t)t, view, wide, box);
+        }
+    }
+    if (queue.n > 0) queue.flush(tab.b, lane, queue.n);
+}
+
+// ---------------------------------------------------------------------------
+// Large triangles
+// ---------------------------------------------------------------------------
+
+// Candidate pixel (x, y) of a set-up triangle: the coverage test of
+// transform.cpp:105-114; on success its depth, for the fragment key.
+// The CPU keeps, per output pixel, the fragment with the largest
+// quality / depth^3 (a later fragment replaces the stored one iff
+// (d/D)^3 * Q < q, transform.cpp:119-142), the earliest in scan order on
+// ties.  The key holds the bits of depth^3 / quality (smaller is better)
+// above the triangle's scan index, so 64-bit atomicMin keeps that winner
+// whatever the scheduling order.
+//
+// The coordinates come from rinv, an approximate reciprocal of den (at most
+// 1 ulp off).  Then l1 and l2 are within 4u|l| of the CPU's n / den
+// (u = 2^-24: 2u from the reciprocal, one rounding here and one in the
+// CPU's division), and l3 = (1 - l1) - l2 within
+// u * (4|l1| + 2|1 - l1| + 4|l2| + 2|l3|) of the CPU's, which is below
+// 21u * M with M = max(|l1|, |l2|, |l3|, 1).  One bound, 24u * M, therefore
+// covers every coordinate: the test is decided when the smallest coordinate
+// is farther than the bound from -1e-6; otherwise the coordinates are
+// recomputed with the reference's divisions.  The depth in the key uses the
+// fast coordinates; the resolve recomputes the winning fragment exactly.
+__device__ __forceinline__ bool test_pixel(const TriSetup& s, float cx, float cy, float za, float zb_, float zc,
+                                           int x, int y, float& d) {
+    const float u = 5.9604645e-8f, eps = 1e-6f;
+    const float tx = __fsub_rn(__fadd_rn((float)x, 0.5f), cx);
+    const float ty = __fsub_rn(__fadd_rn((float)y, 0.5f), cy);
+    const float n1 = __fadd_rn(__fmul_rn(s.b1c1, tx), __fmul_rn(s.c0b0, ty));
+    const float n2 = __fadd_rn(__fmul_rn(s.c1a1, tx), __fmul_rn(s.a0c0, ty));
+    float l1 = __fmul_rn(n1, s.rinv), l2 = __fmul_rn(n2, s.rinv);
+    float l3 = __fsub_rn(__fsub_rn(1.f, l1), l2);
+    const float mn = fminf(fminf(l1, l2), l3);
+    const float M = fmaxf(fmaxf(fabsf(l1), fabsf(l2)), fmaxf(fabsf(l3), 1.f));
+    const float bound = __fmul_rn(24.f * u, M);
+    if (__fadd_rn(mn, bound) < -eps) return false;
+    if (!(__fsub_rn(mn, bound) >= -eps)) {
+        l1 = __fdiv_rn(n1, s.den);
+        l2 = __fdiv_rn(n2, s.den);
+        l3 = __fsub_rn(__fsub_rn(1.f, l1), l2);
+        if (!covered(l1, l2, l3)) return false;
+    }
+    d = interp(za, zb_, zc, l1, l2, l3);
+    return !isnan(d);
+}
+
+// Quality of the key only (the resolve recomputes it exactly): the longest
+// edge in float, a few ulp from the reference's double evaluation.  The
+// squared lengths of an edge shared by two triangles are identical, so
+// equal reference qualities stay equal here.
+__device__ __forceinline__ float key_invq(float4 A, float4 B, float4 C, float precision) {
+    return small_invq(fmaxf(sq2(__fsub_rn(B.x, C.x), __fsub_rn(B.y, C.y)),
+                            fmaxf(sq2(__fsub_rn(A.x, B.x), __fsub_rn(A.y, B.y)),
+                                  sq2(__fsub_rn(A.x, C.x), __fsub_rn(A.y, C.y)))),
+                      precision);
+}
+
+__device__ __forceinline__ unsigned long long frag_key(float d, float invq, uint32_t tri) {
+    uint32_t hi = 0u;
+    if (d > 0.f) hi = __float_as_uint(__fmul_rn(__fmul_rn(__fmul_rn(d, d), d), invq));
+    return ((unsigned long long)hi << 32) | tri;
+}
+
+// One warp rasterises triangle (A, B, C), set up in s with its candidate box:
+// the candidate span of each row, one lane per row and 32 rows at a time,
+// then the spans' pixels flattened over the warp, 32 candidates per round
+// whatever the shape.
+__device__ __forceinline__ void raster_large(const TriSetup& s, float4 A, float4 B, float4 C, float invq,
+                                             uint32_t tri, unsigned long long* z, int wo, int lane) {
+    for (int yb = s.y0; yb <= s.y1; yb += 32) {
+        const int y = yb + lane;
+        int xl = 0, xr = -1;
+        if (y <= s.y1) row_span(s, C.x, C.y, y, xl, xr);
+        const int len = max(0, xr - xl + 1);
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int excl = incl - len;
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int base = 0; base < total; base += 32) {
+            const int c = base + lane;
+            // Row of candidate c: the number of rows whose spans end at
+            // or before c (binary search over the inclusive prefix).
+            int row = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const int probe = __shfl_sync(0xffffffffu, incl, row + step - 1);
+                if (probe <= c) row += step;
+            }
+            const int rxl = __shfl_sync(0xffffffffu, xl, row);
+            const int rex = __shfl_sync(0xffffffffu, excl, row);
+            if (c >= total) continue;
+            const int x = rxl + (c - rex), yy = yb + row;
+            float d;
+            if (test_pixel(s, C.x, C.y, A.z, B.z, C.z, x, yy, d))
+                atomicMin(z + (size_t)yy * wo + x, frag_key(d, invq, tri));
+        }
+    }
+}
+
+// Vertices of triangle `tri` of view V from the stored mesh.
+__device__ __forceinline__ void load_triangle(const DevView& V, uint32_t tri, float4& A, float4& B, float4& C) {
+    const int i = (int)(tri >> V.tri_shift), j = (int)((tri >> 2) & ((1u << (V.tri_shift - 2)) - 1u));
+    int ax, ay, bx, by, cx, cy;
+    tri_vertices(V.w, i, j, (int)(tri & 3u), ax, ay, bx, by, cx, cy);
+    A = __ldg(V.vert + (size_t)ay * V.w + ax);
+    B = __ldg(V.vert + (size_t)by * V.w + bx);
+    C = __ldg(V.vert + (size_t)cy * V.w + cx);
+}
+
+// Grid (CTAs, slots), LARGE_THREADS threads: every warp takes entries of the
+// slot's list in turn.  When the list overflowed (more large triangles than
+// it holds), the warps instead go over all quads of the group's views and
+// rasterise every triangle; those the mesh kernel has done already only
+// repeat keys that are there (atomicMin).
+template <class Tabs>
+__global__ void __launch_bounds__(LARGE_THREADS) large_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
+    grid_dep_wait();
+    const SlotTable& tab = tabs.at(blockIdx.y);
+    const DevTarget& T = tab.t;
+    if (g0 >= T.n_views) return;
+    const int n = tab.b.status->n_large;
+    const int lane = threadIdx.x & 31;
+    const int wid = blockIdx.x * (LARGE_THREADS / 32) + (threadIdx.x >> 5), nw = gridDim.x * (LARGE_THREADS / 32);
+    if (n <= tab.b.large_capacity) {
+        for (int e = wid; e < n; e += nw) {
+            const uint4 q = __ldg(tab.b.large + e);
+            const DevView& V = tab.v[q.y & 255u];
+            float4 A, B, C;
+            load_triangle(V, q.x, A, B, C);
+            TriSetup s;
+            if (!tri_coef(A, B, C, s)) continue;
+            if (q.y & 256u) {
+                if (!tri_range(A, B, C, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, s)) continue;
+            } else {
+                s.x0 = (int)(q.z & 0xffffu);
+                s.x1 = (int)(q.z >> 16);
+                s.y0 = (int)(q.w & 0xffffu);
+                s.y1 = (int)(q.w >> 16);
+            }
+            s.rinv = rcp_approx(s.den);
+            raster_large(s, A, B, C, key_invq(A, B, C, T.precision), q.x, V.z, T.wo, lane);
+        }
+        return;
+    }
+    const bool wrap = T.wrap != 0;
+    for (int view = g0; view < min(T.n_views, g0 + gv); ++view) {
+        const DevView& V = tab.v[view];
+        const int groups = (V.w - 1 + 31) / 32;
+        for (long long g = wid; g < (long long)groups * (V.h - 1); g += nw) {
+            const int i = (int)(g / groups), j0 = (int)(g % groups) * 32, j = j0 + lane;
+            if (T.cull && V.erp_cone && tile_culled(V, T, j0 / WARP_TILE, i / WARP_TILE)) continue;
+            for (int t = 0; t < (wrap ? 4 : 2); ++t) {
+                const uint32_t tri = ((((uint32_t)i << (V.tri_shift - 2)) | (uint32_t)j) << 2) | (uint32_t)t;
+                float4 A, B, C;
+                TriSetup s;
+                bool on = j < V.w - 1 && (t < 2 || j == 0);
+                if (on) {
+                    const float4 v01 = __ldg(V.vert + (size_t)i * V.w + j + 1);
+                    const float4 v10 = __ldg(V.vert + (size_t)(i + 1) * V.w + j);
+                    load_triangle(V, tri, A, B, C);
+                    on = v01.z > 0.f && v10.z > 0.f && v01.x > 0.f && v10.x > 0.f &&
+                         (t >= 2 || (A.z > 0.f && A.x > 0.f)) && tri_coef(A, B, C, s) &&
+                         tri_range(A, B, C, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, s);
+                }
+                for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
+                    const uint32_t k = __shfl_sync(0xffffffffu, tri, __ffs(m) - 1);
+                    float4 a, b, c;
+                    TriSetup r;
+                    load_triangle(V, k, a, b, c);
+                    if (!tri_coef(a, b, c, r) || !tri_range(a, b, c, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, r)) continue;
+                    r.rinv = rcp_approx(r.den);
+                    raster_large(r, a, b, c, key_invq(a, b, c, T.precision), k, V.z, T.wo, lane);
+                }
+            }
+        }
+    }
+}
+
+// Empty keys in the z-buffers of views g0 .. g0 + gv - 1 of every slot, and
+// an empty list of large triangles.  Grid (CTAs, slots).
+template <class Tabs>
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
+    grid_dep_wait();
+    const SlotTable& tab = tabs.at(blockIdx.y);
+    const DevTarget& T = tab.t;
+    if (g0 >= T.n_views) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) tab.b.status->n_large = 0;
+    const size_t n = (size_t)min(gv, T.n_views - g0) * T.wo * T.ho;
+    unsigned long long* z = tab.v[g0].z;  // the group's buffers lie back to back from a 16-byte boundary
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (n & 1)) z[n - 1] = kEmptyKey;
+    for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n / 2; k += (size_t)gridDim.x * 256)
+        reinterpret_cast<ulonglong2*>(z)[k] = make_ulonglong2(kEmptyKey, kEmptyKey);
+}
+
+}  // namespace
+
+template <class Tabs>
+int launch_mesh(const Tabs& tabs, const BatchShape& sh, int g0, cudaStream_t s, cudaEvent_t* ev) {
+    const RasterVariant& rv = kRasterVariants[sh.variant];
+    const int gv = std::min(sh.vg, sh.max_views - g0);
+    const size_t words = (size_t)gv * sh.max_wo * sh.max_ho;
+    if (ev) cudaEventRecord(ev[0], s);
+    launch_dependent(clear_kernel<Tabs>, dim3((unsigned)std::min<size_t>(2048, (words / 2 + 255) / 256 + 1), sh.slots),
+                     dim3(256), 0, s, tabs, g0, gv);
+    const int strips = (sh.max_w - 1 + STRIP - 1) / STRIP + 1;  // and the seam's
+    const dim3 grid((strips + MESH_WARPS - 1) / MESH_WARPS, (sh.max_h - 1 + rv.rows - 1) / rv.rows, sh.slots * gv);
+    switch (rv.small) {
+        case 4: launch_dependent(mesh_kernel<4, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); break;
+        case 8: launch_dependent(mesh_kernel<8, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); break;
+        case 16: launch_dependent(mesh_kernel<16, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); break;
+        default: launch_dependent(mesh_kernel<64, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); break;
+    }
+    if (ev) {
+        cudaEventRecord(ev[1], s);
+        cudaEventRecord(ev[2], s);
+    }
+    launch_dependent(large_kernel<Tabs>, dim3(std::max(1, 148 * 8 / sh.slots), sh.slots), dim3(LARGE_THREADS), 0, s,
+                     tabs, g0, gv);
+    if (ev) cudaEventRecord(ev[3], s);
+    return 3;
+}
+
+template int launch_mesh<TableParam>(const TableParam&, const BatchShape&, int, cudaStream_t, cudaEvent_t*);
+template int launch_mesh<TablePtr>(const TablePtr&, const BatchShape&, int, cudaStream_t, cudaEvent_t*);
+
+}  // namespace rvsb

@@ -83,14 +83,12 @@ cudaError_t scratch_on_current_device(unsigned char** out) {
 // Writes the empty status: no holes, an inverted bounding box.
 __global__ void noalloc_reset_kernel(DevStatus* st) {
     if (threadIdx.x == 0) {
-        st->bin_total = 0;
-        st->bin_overflow = 0;
+        st->n_large = 0;
         st->hole_x0 = INT_MAX;
         st->hole_y0 = INT_MAX;
         st->hole_x1 = INT_MIN;
         st->hole_y1 = INT_MIN;
         st->n_holes = 0;
-        st->pad = 0;
     }
 }
 
