@@ -69,8 +69,9 @@ __device__ __forceinline__ float4 depth_entry(const View& V, int i, int j) {
 }
 
 // L: depth_entry(V, i, j), loaded by the caller (the warp kernel issues a
-// thread's loads ahead of its arithmetic).
-template <class View>
+// thread's loads ahead of its arithmetic).  kErpOut: the output may be
+// equirectangular (compiled out of kernels whose outputs all are perspective).
+template <bool kErpOut, class View>
 __device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T, int i, int j, float4 L) {
     const float d = L.x;
     float x0, x1, x2;
@@ -101,7 +102,7 @@ __device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T,
         y[r] = __fadd_rn(s, V.t[r]);
     }
     float u, v, z;
-    if (T.proj == 1) {
+    if (kErpOut && T.proj == 1) {
         double s2 = 0.0;
         s2 = __dadd_rn(s2, __dmul_rn((double)y[0], (double)y[0]));
         s2 = __dadd_rn(s2, __dmul_rn((double)y[1], (double)y[1]));
@@ -131,10 +132,6 @@ __device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T,
     return make_float4(u, v, z, 0.f);
 }
 
-template <class View>
-__device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T, int i, int j) {
-    return warp_vertex(V, T, i, j, depth_entry(V, i, j));
-}
 
 // Triangle quality of transform.cpp:62-75 (valid_tri): the longest edge by
 // cv::norm (double sum of squared float differences, double sqrt), then
