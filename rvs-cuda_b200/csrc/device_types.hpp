@@ -78,9 +78,7 @@ constexpr int MAX_VIEWS = 16;
 // Status words written by the kernels (device memory, reset per call).
 struct DevStatus {
     int n_large;        // large triangles entered in the list (may exceed its capacity)
-    int hole_x0, hole_y0, hole_x1, hole_y1;   // bounding box of holes (x0 > x1: none)
-    int n_holes;
-    int pad[2];
+    int n_holes;        // nonzero when some pixel is a hole
 };
 
 // Optional intermediate outputs (device pointers, may be null).
@@ -144,15 +142,12 @@ struct SlotBuffers {
     float2* acc01;
     float2* acc23;
     uint64_t* codes;     // Wo*Ho packed output codes + hole bit
-    uint8_t* holes;      // Wo*Ho hole mask (1 = no view covers the pixel)
+    uint32_t* holes;     // hole mask, one bit per pixel (1 = no view covers it), (Wo + 31) / 32 words a row
     uint64_t* scan[4];   // Wo*Ho inpainting scratch each
-    uint64_t* inpaint_seg;  // column-group and warp-segment minima of the inpainting pre-passes
+    uint64_t* inpaint_sum;  // column minima of the inpainting's row groups
     float4* pcolor;      // Precision != 1: blended colour per raster pixel
     int32_t* psrc;       // Precision != 1: inpainting source of every hole
 };
-
-// Most row groups per column strip in the inpainting passes.
-constexpr int INPAINT_MAX_GROUPS = 8;
 
 // Everything one synthesis (one virtual view) needs on the device.  A batch
 // keeps one table per slot in device memory; every kernel of the batch reads

@@ -60,7 +60,7 @@ RasterDims raster_dims(const rvsb_camera& virt, const rvsb_synth_params& p) {
 namespace {
 
 struct SlotNeeds {
-    size_t vert, out, large;
+    size_t vert, out, large, hole_words, sum_words;
 };
 
 SlotNeeds needs_of(const rvsb_scene* sc, int wo, int ho) {
@@ -69,6 +69,8 @@ SlotNeeds needs_of(const rvsb_scene* sc, int wo, int ho) {
     n.out = (size_t)wo * ho;
     // About 1% of the triangles of an unmagnified view are large; when they
     // do not fit, large_kernel goes over the whole mesh.
+    n.hole_words = (size_t)((wo + 31) / 32) * ho;
+    n.sum_words = inpaint_sum_words(wo, ho);
     n.large = std::min<size_t>(INT32_MAX / 2, std::max<size_t>(1 << 14, n.vert / 11));
     return n;
 }
@@ -77,8 +79,8 @@ SlotNeeds needs_of(const rvsb_scene* sc, int wo, int ho) {
 
 size_t SlotWorkspace::bytes_for(const rvsb_scene* sc, int wo, int ho, bool rescale) {
     const SlotNeeds n = needs_of(sc, wo, ho);
-    return sizeof(DevStatus) + n.vert * sizeof(float4) + n.large * sizeof(uint4) + n.out * (sizeof(uint64_t) * 5 + 1) +
-           inpaint_seg_words(wo) * sizeof(uint64_t) + (rescale ? n.out * (sizeof(float4) + 2 * sizeof(int32_t)) : 0);
+    return sizeof(DevStatus) + n.vert * sizeof(float4) + n.large * sizeof(uint4) + n.out * sizeof(uint64_t) * 5 +
+           n.hole_words * sizeof(uint32_t) + n.sum_words * sizeof(uint64_t) + (rescale ? n.out * (sizeof(float4) + 2 * sizeof(int32_t)) : 0);
 }
 
 void SlotWorkspace::ensure_rescale(rvsb_context* ctx, int wo, int ho) {
@@ -101,14 +103,16 @@ void SlotWorkspace::ensure(rvsb_context* ctx, const rvsb_scene* sc, int wo, int 
         large.alloc(ctx, n.large * sizeof(uint4));
         cap_large = n.large;
     }
-    const size_t seg_words = inpaint_seg_words(wo);
-    if (seg_words > cap_seg_words) {
-        inpaint_seg.alloc(ctx, seg_words * sizeof(uint64_t));
-        cap_seg_words = seg_words;
+    if (n.hole_words > cap_hole_words) {
+        holes.alloc(ctx, n.hole_words * sizeof(uint32_t));
+        cap_hole_words = n.hole_words;
+    }
+    if (n.sum_words > cap_sum_words) {
+        inpaint_sum.alloc(ctx, n.sum_words * sizeof(uint64_t));
+        cap_sum_words = n.sum_words;
     }
     if (n.out > cap_out) {
         codes.alloc(ctx, n.out * sizeof(uint64_t));
-        holes.alloc(ctx, n.out);
         scan.alloc(ctx, 4 * n.out * sizeof(uint64_t));
         cap_out = n.out;
     }
@@ -305,11 +309,11 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     B.large = ws.large.as<uint4>();
     B.large_capacity = (int)ws.cap_large;
     B.codes = ws.codes.as<uint64_t>();
-    B.holes = ws.holes.as<uint8_t>();
+    B.holes = ws.holes.as<uint32_t>();
     for (int s = 0; s < 4; ++s) B.scan[s] = ws.scan.as<uint64_t>() + (size_t)s * npix;
     B.acc01 = reinterpret_cast<float2*>(B.scan[3]);
     B.acc23 = reinterpret_cast<float2*>(B.codes);
-    B.inpaint_seg = ws.inpaint_seg.as<uint64_t>();
+    B.inpaint_sum = ws.inpaint_sum.as<uint64_t>();
     if (rd.rescale) {
         B.pcolor = ws.pcolor.as<float4>();
         B.psrc = r.dbg.inpaint_source ? r.dbg.inpaint_source : ws.psrc.as<int32_t>();

@@ -131,14 +131,14 @@ void launch_tile_depth(const TileDepthJobs& jobs, int n, int max_w, int max_h, c
 void launch_decode_color(const uint16_t* y, const uint16_t* u, const uint16_t* v, int w, int h, uint64_t* out,
                          cudaStream_t s);
 
-// Inpainting of one image outside a batch (no slot table): the scans over
-// `holes` with caller-provided scratch (status, codes and four scan buffers
-// of w*h words each); the chosen source of every hole goes to `sources`.
-// Words of a slot's inpainting column-minima table for outputs up to wo
-// wide (group minima and warp-segment minima of the column pre-passes).
-size_t inpaint_seg_words(int wo);
+// Words of the column minima of the inpainting's row groups.
+size_t inpaint_sum_words(int wo, int ho);
 
-void launch_inpaint_scans(DevStatus* st, const uint8_t* holes, uint64_t* codes, uint64_t* const scan[4], int w,
-                          int h, int32_t* sources, cudaStream_t s);
+// Inpainting sources of one image outside a batch (no slot table): hole bits
+// as SlotBuffers::holes (bits beyond the width set), four scan buffers of
+// w*h words and inpaint_sum_words words of scratch; the source of every hole
+// goes to `sources`.
+void launch_inpaint_sources(const DevStatus* st, const uint32_t* holes, uint64_t* const scan[4], uint64_t* sum, int w,
+                            int h, int32_t* sources, cudaStream_t s);
 
 }  // namespace rvsb

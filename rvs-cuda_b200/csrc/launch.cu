@@ -27,10 +27,6 @@ __global__ void slot_init_kernel(const __grid_constant__ Tabs tabs) {
     if (threadIdx.x == 0) {
         DevStatus* st = tabs.at(blockIdx.x).b.status;
         st->n_large = 0;
-        st->hole_x0 = INT_MAX;
-        st->hole_y0 = INT_MAX;
-        st->hole_x1 = INT_MIN;
-        st->hole_y1 = INT_MIN;
         st->n_holes = 0;
     }
 }

@@ -22,7 +22,7 @@
 //    code on that device).  Make that first call before any stream capture
 //    begins; later calls only launch kernels.
 //  - Initial contents: nothing in the array needs to start at zero.  The
-//    status block (hole count and hole bounding box) must start each call
+//    status block (whether there are holes) must start each call
 //    empty, and the first kernel of every call writes it so; every scan word
 //    a later kernel reads has been written earlier in the same call.
 //  - All calls on one device share the one array: two calls whose kernels
@@ -43,7 +43,11 @@ namespace {
 
 constexpr size_t kMaxPixels = size_t(1) << 19;
 constexpr size_t kStatusBytes = 256;
-constexpr size_t kWordsPerPixel = 5;  // codes + 4 scan buffers
+// 4 scan buffers, and one word more for the row groups' minima and the hole
+// bits: 3 words per column and group (at most 1 + h / 32 groups of 32 rows,
+// so at most 3 * (w + 2^19 / 32) words, 147,456) and half a word per 32
+// columns or less (at most 2^16 half words for images 2 pixels wide).
+constexpr size_t kWordsPerPixel = 5;
 constexpr size_t kScratchBytes = kStatusBytes + kWordsPerPixel * sizeof(uint64_t) * kMaxPixels;
 constexpr int kMaxDevices = 64;
 
@@ -80,56 +84,34 @@ cudaError_t scratch_on_current_device(unsigned char** out) {
     return cudaSuccess;
 }
 
-// Writes the empty status: no holes, an inverted bounding box.
+// Writes the empty status: no holes.
 __global__ void noalloc_reset_kernel(DevStatus* st) {
     if (threadIdx.x == 0) {
         st->n_large = 0;
-        st->hole_x0 = INT_MAX;
-        st->hole_y0 = INT_MAX;
-        st->hole_x1 = INT_MIN;
-        st->hole_y1 = INT_MIN;
         st->n_holes = 0;
     }
 }
 
-// Per pixel: the code word the fill copies (only the hole bit: no colour is
-// carried), the source of a non-hole (itself; -1 marks a hole until the fill
-// writes it) and the hole count and bounding box, one atomic per warp.
+// The hole mask as bits, one warp per mask word (bits beyond the width set),
+// the source of every pixel that is no hole (itself; -1 marks a hole until
+// the fill writes it), and whether there is a hole.
 __global__ void noalloc_prep_kernel(const uint8_t* __restrict__ holes, int w, int h, DevStatus* st,
-                                    uint64_t* __restrict__ codes, int32_t* __restrict__ sources) {
-    const size_t n = (size_t)w * h;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t base = (size_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const size_t o = base + threadIdx.x;
-        int x0 = INT_MAX, y0 = INT_MAX, x1 = INT_MIN, y1 = INT_MIN;
+                                    uint32_t* __restrict__ bits, int32_t* __restrict__ sources) {
+    const int words = (w + 31) / 32, lane = threadIdx.x & 31;
+    const int stride = gridDim.x * (blockDim.x >> 5);
+    for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < words * h; k += stride) {
+        const int y = k / words, x = (k % words) * 32 + lane;
         bool hole = false;
-        if (o < n) {
-            const int x = (int)(o % (size_t)w), y = (int)(o / (size_t)w);
+        if (x < w) {
+            const size_t o = (size_t)y * w + x;
             hole = holes[o] != 0;
-            codes[o] = hole ? dev::kHoleBit : 0ull;
             sources[o * 2 + 0] = hole ? -1 : x;
             sources[o * 2 + 1] = hole ? -1 : y;
-            if (hole) {
-                x0 = x1 = x;
-                y0 = y1 = y;
-            }
         }
-        const unsigned mask = __ballot_sync(0xffffffffu, hole);
-        if (mask) {
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) {
-                x0 = min(x0, __shfl_xor_sync(0xffffffffu, x0, s));
-                y0 = min(y0, __shfl_xor_sync(0xffffffffu, y0, s));
-                x1 = max(x1, __shfl_xor_sync(0xffffffffu, x1, s));
-                y1 = max(y1, __shfl_xor_sync(0xffffffffu, y1, s));
-            }
-            if ((threadIdx.x & 31) == 0) {
-                atomicMin(&st->hole_x0, x0);
-                atomicMin(&st->hole_y0, y0);
-                atomicMax(&st->hole_x1, x1);
-                atomicMax(&st->hole_y1, y1);
-                atomicAdd(&st->n_holes, __popc(mask));
-            }
+        const unsigned mask = __ballot_sync(0xffffffffu, hole), beyond = __ballot_sync(0xffffffffu, x >= w);
+        if (lane == 0) {
+            bits[k] = mask | beyond;
+            if (mask) st->n_holes = 1;
         }
     }
 }
@@ -172,9 +154,10 @@ extern "C" rvsb_status rvsb_inpaint_sources_noalloc(const uint8_t* holes, int wi
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     DevStatus* st = reinterpret_cast<DevStatus*>(base);
     uint64_t* words = reinterpret_cast<uint64_t*>(base + kStatusBytes);
-    uint64_t* codes = words;
     uint64_t* scan[4];
-    for (int k = 0; k < 4; ++k) scan[k] = words + (size_t)(k + 1) * (size_t)npix;
+    for (int k = 0; k < 4; ++k) scan[k] = words + (size_t)k * (size_t)npix;
+    uint64_t* sum = words + 4 * kMaxPixels;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(sum + inpaint_sum_words(width, height));
     noalloc_reset_kernel<<<1, 32, 0, s>>>(st);
     int dev = 0, sms = 0;
     e = cudaGetDevice(&dev);
@@ -185,8 +168,8 @@ extern "C" rvsb_status rvsb_inpaint_sources_noalloc(const uint8_t* holes, int wi
     }
     const int threads = 256;
     const int blocks = (int)std::min<long long>((npix + threads - 1) / threads, (long long)sms * 8);
-    noalloc_prep_kernel<<<blocks, threads, 0, s>>>(holes, width, height, st, codes, sources);
-    launch_inpaint_scans(st, holes, codes, scan, width, height, sources, s);
+    noalloc_prep_kernel<<<blocks, threads, 0, s>>>(holes, width, height, st, bits, sources);
+    launch_inpaint_sources(st, bits, scan, sum, width, height, sources, s);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error(err, err_len, "kernel launch failed: %s", cudaGetErrorString(e));

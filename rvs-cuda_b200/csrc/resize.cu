@@ -14,12 +14,12 @@ using namespace dev;
 
 struct Filled {
     const float4* color;
-    const uint8_t* holes;
+    const uint32_t* holes;  // one bit per pixel
     const int32_t* src;
     int w;
     __device__ __forceinline__ float3 at(int x, int y) const {
         size_t o = (size_t)y * w + x;
-        if (holes[o]) o = (size_t)src[o * 2 + 1] * w + src[o * 2 + 0];
+        if (holes[(size_t)y * ((w + 31) / 32) + (x >> 5)] >> (x & 31) & 1u) o = (size_t)src[o * 2 + 1] * w + src[o * 2 + 0];
         const float4 c = color[o];
         return make_float3(c.x, c.y, c.z);
     }

@@ -102,7 +102,6 @@ __global__ void __launch_bounds__(TILE_W * TILE_H) resolve_kernel(const __grid_c
         code = (uint64_t)quantize(a.c0, T.max_val) | ((uint64_t)quantize(a.c1, T.max_val) << 16) |
                ((uint64_t)quantize(a.c2, T.max_val) << 32) | (hole ? kHoleBit : 0ull);
         tab.b.codes[po] = code;
-        tab.b.holes[po] = hole ? 1 : 0;
         if (T.rescale) tab.b.pcolor[po] = make_float4(a.c0, a.c1, a.c2, 0.f);
         if (Extras) {
             const DebugPtrs& dbg = tab.dbg;
@@ -139,16 +138,14 @@ __global__ void __launch_bounds__(TILE_W * TILE_H) resolve_kernel(const __grid_c
             }
         }
     }
-    if (hm && lane == 0) {
-        // Bounding box of the holes, from the warp's mask (two rows of 16).
-        const unsigned cols = (hm | (hm >> 16)) & 0xffffu;
-        DevStatus* st = tab.b.status;
-        atomicMin(&st->hole_x0, x + __ffs(cols) - 1);
-        atomicMax(&st->hole_x1, x + 31 - __clz(cols));
-        atomicMin(&st->hole_y0, (hm & 0xffffu) ? y : y + 1);
-        atomicMax(&st->hole_y1, (hm >> 16) ? y + 1 : y);
-        atomicAdd(&st->n_holes, 1);
+    // Hole bits, 16 columns of each of the warp's two rows; those beyond the
+    // width are set.
+    const unsigned bits = hm | __ballot_sync(0xffffffffu, x >= T.wo);
+    if (!(lane & 15) && y < T.ho) {
+        const int words = (T.wo + 31) / 32;
+        reinterpret_cast<uint16_t*>(tab.b.holes + (size_t)y * words)[x >> 4] = (uint16_t)(bits >> (lane & 16));
     }
+    if (hm && lane == 0) tab.b.status->n_holes = 1;
 }
 
 }  // namespace
