@@ -19,9 +19,18 @@ namespace {
 using namespace dev;
 
 constexpr int MS_THREADS = 256;
+constexpr int MS_WARPS = MS_THREADS / 32;
+constexpr int MS_CHUNKS = 8;   // 32-column chunks a warp holds at once
+constexpr int MS_COLS = 128;   // columns per CTA of the column windows
+constexpr int MS_ROWS = 64;    // rows a thread of it slides over
+constexpr int MS_BATCH = 8;    // of them loaded together
 
 // Row-window sums of masked luma: one CTA per (row, view, slot).  The row's
-// exclusive prefix (double sums, integer counts) is built in shared memory.
+// exclusive prefix (double sums, integer counts) is built in shared memory:
+// each warp scans MS_CHUNKS chunks of 32 columns, loaded together and
+// coalesced, the warps' totals are added, and wide rows take several rounds.
+// (With a run of consecutive columns per thread, read twice, 16 bytes every
+// 128, the kernel took 162 us on 4 views of 1920x1080.)
 template <class Tabs>
 __global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_constant__ Tabs tabs) {
     grid_dep_wait();
@@ -35,61 +44,75 @@ __global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_consta
     const int w = T.wo;
     double* P = reinterpret_cast<double*>(s_raw);                     // w + 1 prefix sums
     int* C = reinterpret_cast<int*>(s_raw + sizeof(double) * (w + 1));  // w + 1 prefix counts
-    __shared__ double s_wsum[MS_THREADS / 32];
-    __shared__ int s_wcnt[MS_THREADS / 32];
+    __shared__ double s_wsum[MS_WARPS];
+    __shared__ int s_wcnt[MS_WARPS];
     const size_t npo = (size_t)T.wo * T.ho;
     const float4* row = M.view + (size_t)v * npo + (size_t)y * w;
-    // Each thread sums a contiguous chunk, then a block scan of the chunks.
-    const int per = (w + MS_THREADS - 1) / MS_THREADS;
-    const int beg = min(w, (int)threadIdx.x * per), end = min(w, beg + per);
-    double ls = 0.0;
-    int lc = 0;
-    for (int x = beg; x < end; ++x) {
-        const float4 c = row[x];
-        if (c.w > 0.f && isfinite(c.x)) {
-            ls += (double)c.x;
-            ++lc;
-        }
-    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double is = ls;
-    int ic = lc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double a = __shfl_up_sync(0xffffffffu, is, o);
-        const int b = __shfl_up_sync(0xffffffffu, ic, o);
-        if (lane >= o) {
-            is += a;
-            ic += b;
-        }
-    }
-    if (lane == 31) {
-        s_wsum[warp] = is;
-        s_wcnt[warp] = ic;
-    }
-    __syncthreads();
     double base = 0.0;
     int cbase = 0;
-    for (int k = 0; k < warp; ++k) {
-        base += s_wsum[k];
-        cbase += s_wcnt[k];
-    }
-    double run = base + is - ls;
-    int crun = cbase + ic - lc;
     if (threadIdx.x == 0) {
         P[0] = 0.0;
         C[0] = 0;
     }
-    for (int x = beg; x < end; ++x) {
-        const float4 c = row[x];
-        if (c.w > 0.f && isfinite(c.x)) {
-            run += (double)c.x;
-            ++crun;
+    for (int r0 = 0; r0 < w; r0 += MS_THREADS * MS_CHUNKS) {
+        const int x0 = r0 + warp * 32 * MS_CHUNKS + lane;
+        double s[MS_CHUNKS];
+        unsigned mask[MS_CHUNKS];
+#pragma unroll
+        for (int k = 0; k < MS_CHUNKS; ++k) {
+            const int x = x0 + 32 * k;
+            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (x < w) c = row[x];
+            const bool in = c.w > 0.f && isfinite(c.x);
+            mask[k] = __ballot_sync(0xffffffffu, in);
+            s[k] = in ? (double)c.x : 0.0;
         }
-        P[x + 1] = run;
-        C[x + 1] = crun;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (int k = 0; k < MS_CHUNKS; ++k) {
+                const double a = __shfl_up_sync(0xffffffffu, s[k], o);
+                if (lane >= o) s[k] += a;
+            }
+        }
+        double run = 0.0;
+        int crun = 0;
+        int cnt[MS_CHUNKS];
+#pragma unroll
+        for (int k = 0; k < MS_CHUNKS; ++k) {
+            const double t = __shfl_sync(0xffffffffu, s[k], 31);
+            s[k] += run;
+            cnt[k] = crun + __popc(mask[k] & (0xffffffffu >> (31 - lane)));
+            run += t;
+            crun += __popc(mask[k]);
+        }
+        if (lane == 0) {
+            s_wsum[warp] = run;
+            s_wcnt[warp] = crun;
+        }
+        __syncthreads();
+        double before = base;
+        int cbefore = cbase;
+#pragma unroll
+        for (int k = 0; k < MS_WARPS; ++k) {
+            if (k < warp) {
+                before += s_wsum[k];
+                cbefore += s_wcnt[k];
+            }
+            base += s_wsum[k];
+            cbase += s_wcnt[k];
+        }
+#pragma unroll
+        for (int k = 0; k < MS_CHUNKS; ++k) {
+            const int x = x0 + 32 * k;
+            if (x < w) {
+                P[x + 1] = before + s[k];
+                C[x + 1] = cbefore + cnt[k];
+            }
+        }
+        __syncthreads();
     }
-    __syncthreads();
     const int rad = M.rad;
     double* hs = M.hsum + (size_t)v * npo + (size_t)y * w;
     int* hc = M.hcnt + (size_t)v * npo + (size_t)y * w;
@@ -100,75 +123,90 @@ __global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_consta
     }
 }
 
-// Column windows of the row sums, one thread per column and view, sliding
-// down the column; writes the blurred luma.
+// Column windows of the row sums: a thread per column and view slides over
+// MS_ROWS rows, from a window summed up anew.  At 1080 rows and a radius of
+// 54 that reads each row sum 3.7 times instead of twice, but runs 17 times as
+// many threads, and the loads of MS_BATCH rows are in flight together: 54 us
+// on 4 views of 1920x1080 against 827 us with one thread per whole column
+// (60 CTAs of 128 threads on 148 SMs); 32 and 128 rows: 64 and 62 us.
+// Writes the blurred luma.
+// Grid (ceil(max_wo / MS_COLS) * segments, views, slots).
 template <class Tabs>
-__global__ void ms_cols_kernel(const __grid_constant__ Tabs tabs) {
+__global__ void __launch_bounds__(MS_COLS) ms_cols_kernel(const __grid_constant__ Tabs tabs, int segments) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z);
     const MsPtrs& M = tab.ms;
     if (!M.on) return;
     const DevTarget& T = tab.t;
-    const int v = blockIdx.y, x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= T.n_views || x >= T.wo) return;
+    const int v = blockIdx.y, x = blockIdx.x / segments * MS_COLS + threadIdx.x;
     const int w = T.wo, h = T.ho, rad = M.rad;
+    const int y0 = (int)(blockIdx.x % segments) * MS_ROWS, y1 = min(h, y0 + MS_ROWS);
+    if (v >= T.n_views || x >= w || y0 >= h) return;
     const size_t npo = (size_t)w * h;
-    const double* hs = M.hsum + (size_t)v * npo;
-    const int* hc = M.hcnt + (size_t)v * npo;
-    const float4* vw = M.view + (size_t)v * npo;
-    float* out = M.blur + (size_t)v * npo;
+    const double* hs = M.hsum + (size_t)v * npo + x;
+    const int* hc = M.hcnt + (size_t)v * npo + x;
+    float* out = M.blur + (size_t)v * npo + x;
     double s = 0.0;
     int c = 0;
-    for (int y = 0; y <= min(rad, h - 1); ++y) {
-        s += hs[(size_t)y * w + x];
-        c += hc[(size_t)y * w + x];
+    const int ya = max(0, y0 - rad), yb = min(h - 1, y0 + rad);
+#pragma unroll 8
+    for (int y = ya; y <= yb; ++y) {
+        s += __ldg(hs + (size_t)y * w);
+        c += __ldg(hc + (size_t)y * w);
     }
-    for (int y = 0; y < h; ++y) {
-        const size_t o = (size_t)y * w + x;
-        float b = 0.f;
-        if (vw[o].w > 0.f && c > 0) {
-            const unsigned sum = (unsigned)(int)s;
-            b = __fdiv_rn((float)sum, (float)c);
+    // The rows entering and leaving the window, MS_BATCH at a time, before
+    // the sums that wait for them.
+    for (int yb0 = y0; yb0 < y1; yb0 += MS_BATCH) {
+        double sin[MS_BATCH], sout[MS_BATCH];
+        int cin[MS_BATCH], cout[MS_BATCH];
+#pragma unroll
+        for (int k = 0; k < MS_BATCH; ++k) {
+            const int yin = yb0 + k + rad + 1, yout = yb0 + k - rad;
+            const bool i = yin < h, o = yout >= 0 && yout < h;
+            sin[k] = i ? __ldg(hs + (size_t)yin * w) : 0.0;
+            cin[k] = i ? __ldg(hc + (size_t)yin * w) : 0;
+            sout[k] = o ? __ldg(hs + (size_t)yout * w) : 0.0;
+            cout[k] = o ? __ldg(hc + (size_t)yout * w) : 0;
         }
-        out[o] = b;
-        const int yin = y + rad + 1, yout = y - rad;
-        if (yin < h) {
-            s += hs[(size_t)yin * w + x];
-            c += hc[(size_t)yin * w + x];
-        }
-        if (yout >= 0) {
-            s -= hs[(size_t)yout * w + x];
-            c -= hc[(size_t)yout * w + x];
+#pragma unroll
+        for (int k = 0; k < MS_BATCH; ++k) {
+            if (yb0 + k < y1) out[(size_t)(yb0 + k) * w] = c > 0 ? __fdiv_rn((float)(unsigned)(int)s, (float)c) : 0.f;
+            s += sin[k];
+            c += cin[k];
+            s -= sout[k];
+            c -= cout[k];
         }
     }
 }
 
-// The two bands' blends per pixel, added; one thread per 2x2 output block
-// rewrites the colour part of the codes (the hole bits from the raster stay)
-// and the output samples of hole-free blocks.
+constexpr int MS_TILE_W = 32, MS_TILE_H = 8;
+
+// The two bands' blends per pixel, added: rewrites the colour part of the
+// codes (the holes stay the raster's) and the output samples of hole-free 2x2
+// blocks.  One thread per pixel, a warp 16 x 2 of them (the lanes of a chroma
+// block exchange its samples).  Grid (ceil(max_wo / 32), ceil(max_ho / 8),
+// slots).
 template <class Tabs>
-__global__ void ms_blend_kernel(const __grid_constant__ Tabs tabs) {
+__global__ void __launch_bounds__(MS_TILE_W * MS_TILE_H) ms_blend_kernel(const __grid_constant__ Tabs tabs) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z);
     const MsPtrs& M = tab.ms;
     if (!M.on) return;
     const DevTarget& T = tab.t;
-    const int bx = blockIdx.x * blockDim.x + threadIdx.x, by = blockIdx.y;
-    const int x0 = 2 * bx, y0 = 2 * by;
-    if (x0 >= T.wo || y0 >= T.ho) return;
-    const size_t npo = (size_t)T.wo * T.ho;
-    uint64_t code[4];
-    bool any_hole = false;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        code[p] = 0;
-        // partial blocks of a raster of odd width or height (Precision != 1)
-        if (x0 + (p & 1) >= T.wo || y0 + (p >> 1) >= T.ho) continue;
-        const size_t o = (size_t)(y0 + (p >> 1)) * T.wo + x0 + (p & 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * MS_TILE_W + (warp & 1) * 16 + (lane & 15);
+    const int y = blockIdx.y * MS_TILE_H + (warp >> 1) * 2 + (lane >> 4);
+    const bool inside = x < T.wo && y < T.ho;
+    const size_t npo = (size_t)T.wo * T.ho, o = inside ? (size_t)y * T.wo + x : 0;
+    uint64_t code = 0;
+    bool hole = false;
+    if (inside) {
         BlendAcc lo = {0.f, 0.f, 0.f, 0.f}, hi = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
         for (int v = 0; v < T.n_views; ++v) {
             const float4 c = M.view[(size_t)v * npo + o];
-            const float b = M.blur[(size_t)v * npo + o];
+            // 0 outside the mask of quality > 0
+            const float b = c.w > 0.f ? M.blur[(size_t)v * npo + o] : 0.f;
             const float3 lowc = make_float3(b, c.y, c.z);
             const float3 highc = make_float3(__fsub_rn(c.x, b), __fsub_rn(c.y, c.y), __fsub_rn(c.z, c.z));
             blend_view(lo, v, lowc, c.w, M.low_exp, M.low_int, M.low_exp < 0.f);
@@ -176,32 +214,31 @@ __global__ void ms_blend_kernel(const __grid_constant__ Tabs tabs) {
         }
         const float f0 = __fadd_rn(lo.c0, hi.c0), f1 = __fadd_rn(lo.c1, hi.c1), f2 = __fadd_rn(lo.c2, hi.c2);
         if (T.rescale) tab.b.pcolor[o] = make_float4(f0, f1, f2, 0.f);
-        const uint64_t hole = tab.b.codes[o] & kHoleBit;
-        any_hole |= hole != 0;
-        code[p] = (uint64_t)quantize(f0, T.max_val) | ((uint64_t)quantize(f1, T.max_val) << 16) |
-                  ((uint64_t)quantize(f2, T.max_val) << 32) | hole;
-        tab.b.codes[o] = code[p];
+        hole = tab.b.holes[(size_t)y * ((T.wo + 31) / 32) + (x >> 5)] >> (x & 31) & 1u;
+        code = (uint64_t)quantize(f0, T.max_val) | ((uint64_t)quantize(f1, T.max_val) << 16) |
+               ((uint64_t)quantize(f2, T.max_val) << 32) | (hole ? kHoleBit : 0ull);
+        tab.b.codes[o] = code;
         if (tab.dbg.blend_color) {
             tab.dbg.blend_color[o * 3 + 0] = f0;
             tab.dbg.blend_color[o * 3 + 1] = f1;
             tab.dbg.blend_color[o * 3 + 2] = f2;
         }
     }
-    if (any_hole || T.rescale) return;  // written by the inpainting passes or the resize
-    const size_t o = (size_t)y0 * T.wo + x0;
-    tab.out_y[o] = (uint16_t)(code[0] & 0xffff);
-    tab.out_y[o + 1] = (uint16_t)(code[1] & 0xffff);
-    tab.out_y[o + T.wo] = (uint16_t)(code[2] & 0xffff);
-    tab.out_y[o + T.wo + 1] = (uint16_t)(code[3] & 0xffff);
-    uint32_t su = 0, sv = 0;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        su += (uint32_t)((code[p] >> 16) & 0xffff);
-        sv += (uint32_t)((code[p] >> 32) & 0xffff);
+    if (T.rescale) return;  // written by the resize
+    const unsigned hm = __ballot_sync(0xffffffffu, hole);
+    uint32_t su = (uint32_t)(code >> 16) & 0xffffu, sv = (uint32_t)(code >> 32) & 0xffffu;
+    su += __shfl_xor_sync(0xffffffffu, su, 1);
+    sv += __shfl_xor_sync(0xffffffffu, sv, 1);
+    su += __shfl_xor_sync(0xffffffffu, su, 16);
+    sv += __shfl_xor_sync(0xffffffffu, sv, 16);
+    // Blocks with holes are the inpainting's.
+    if (!inside || (hm & (0x00030003u << (lane & 14)))) return;
+    tab.out_y[o] = (uint16_t)(code & 0xffff);
+    if (!(lane & 17)) {
+        const size_t co = (size_t)(y / 2) * (T.wo / 2) + x / 2;
+        tab.out_u[co] = quarter_round(su, T.chroma_ties_up);
+        tab.out_v[co] = quarter_round(sv, T.chroma_ties_up);
     }
-    const size_t co = (size_t)by * (T.wo / 2) + bx;
-    tab.out_u[co] = quarter_round(su, T.chroma_ties_up);
-    tab.out_v[co] = quarter_round(sv, T.chroma_ties_up);
 }
 
 }  // namespace
@@ -210,9 +247,11 @@ template <class Tabs>
 int launch_ms(const Tabs& tabs, const BatchShape& sh, cudaStream_t s) {
     const size_t smem = (sizeof(double) + sizeof(int)) * (size_t)(sh.max_wo + 1);
     launch_dependent(ms_rows_kernel<Tabs>, dim3(sh.max_ho, sh.max_views, sh.slots), dim3(MS_THREADS), smem, s, tabs);
-    launch_dependent(ms_cols_kernel<Tabs>, dim3((sh.max_wo + 127) / 128, sh.max_views, sh.slots), dim3(128), 0, s, tabs);
-    launch_dependent(ms_blend_kernel<Tabs>, dim3(((sh.max_wo + 1) / 2 + 127) / 128, (sh.max_ho + 1) / 2, sh.slots),
-                     dim3(128), 0, s, tabs);
+    const int segments = (sh.max_ho + MS_ROWS - 1) / MS_ROWS;
+    launch_dependent(ms_cols_kernel<Tabs>, dim3((sh.max_wo + MS_COLS - 1) / MS_COLS * segments, sh.max_views, sh.slots),
+                     dim3(MS_COLS), 0, s, tabs, segments);
+    launch_dependent(ms_blend_kernel<Tabs>, dim3((sh.max_wo + MS_TILE_W - 1) / MS_TILE_W, (sh.max_ho + MS_TILE_H - 1) / MS_TILE_H, sh.slots),
+                     dim3(MS_TILE_W * MS_TILE_H), 0, s, tabs);
     return 3;
 }
 
