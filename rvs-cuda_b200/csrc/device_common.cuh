@@ -309,9 +309,27 @@ __device__ __forceinline__ float3 input_color(const DevView& V, int x, int y) {
 __device__ __forceinline__ float blend_pow(float x, float e, int e_int) {
     if (e == 1.f) return x;
     if (e_int > 0) {
+        // e_int - 1 multiplications: the exponent is the same for all pixels,
+        // so the jump is uniform.
         const double b = (double)x;
         double r = b;
-        for (int k = 1; k < e_int; ++k) r = __dmul_rn(r, b);
+        switch (e_int) {
+            case 16: r = __dmul_rn(r, b); [[fallthrough]];
+            case 15: r = __dmul_rn(r, b); [[fallthrough]];
+            case 14: r = __dmul_rn(r, b); [[fallthrough]];
+            case 13: r = __dmul_rn(r, b); [[fallthrough]];
+            case 12: r = __dmul_rn(r, b); [[fallthrough]];
+            case 11: r = __dmul_rn(r, b); [[fallthrough]];
+            case 10: r = __dmul_rn(r, b); [[fallthrough]];
+            case 9: r = __dmul_rn(r, b); [[fallthrough]];
+            case 8: r = __dmul_rn(r, b); [[fallthrough]];
+            case 7: r = __dmul_rn(r, b); [[fallthrough]];
+            case 6: r = __dmul_rn(r, b); [[fallthrough]];
+            case 5: r = __dmul_rn(r, b); [[fallthrough]];
+            case 4: r = __dmul_rn(r, b); [[fallthrough]];
+            case 3: r = __dmul_rn(r, b); [[fallthrough]];
+            default: r = __dmul_rn(r, b);
+        }
         return __double2float_rn(r);
     }
     return powf(x, e);

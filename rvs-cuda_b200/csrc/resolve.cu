@@ -6,6 +6,13 @@
 // One thread per pixel; a warp covers 16 x 2 pixels, so a 2x2 chroma block
 // is four of its lanes, and a CTA 32 x 8, whose fragments share vertices and
 // colours through L1.
+//
+// Bound by instruction issue and the latency of the gathers (three vertices,
+// three colours per pixel and view) together: 4 views of 1920x1080 take 111
+// us (8.3 M pixel-views; their keys, vertices and colours, each read once,
+// are 265 MB, 41 us), 105 us a view in a batch of 8.  Five CTAs per SM at 48
+// registers beat four at 64 (batch 107 against 117 us), two views' gathers in
+// flight per thread (116) and six CTAs at 40 registers (112).
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -19,12 +26,22 @@ using namespace dev;
 
 constexpr int TILE_W = 32, TILE_H = 8;
 
+// The fields of a view the resolve reads.
+struct __align__(16) ResolveView {
+    const float4* vert;
+    const uint64_t* color;
+    const unsigned long long* z;
+    int w, tri_shift;
+    float color_scale;
+    int pad;
+};
+
 // Grid (ceil(max_wo / 32), ceil(max_ho / 8), slots): views g0 .. g0 + gv - 1
 // of every slot; the last group of a slot's views writes its output, earlier
 // ones keep the running blend in acc01 / acc23.  Extras: the per-view
 // multispectral, auxiliary and debug outputs are written.
 template <bool Extras, class Tabs>
-__global__ void __launch_bounds__(TILE_W * TILE_H) resolve_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
+__global__ void __launch_bounds__(TILE_W * TILE_H, 5) resolve_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z);
     const DevTarget& T = tab.t;
@@ -35,6 +52,14 @@ __global__ void __launch_bounds__(TILE_W * TILE_H) resolve_kernel(const __grid_c
     if (blockIdx.x * TILE_W >= T.wo || blockIdx.y * TILE_H >= T.ho) return;
     const bool inside = x < T.wo && y < T.ho;
     const int g1 = min(T.n_views, g0 + gv);
+    // The views' fields once per CTA, in shared memory: the table is indexed by
+    // a loop variable, so each use of it would be a load of its own.
+    __shared__ ResolveView s_view[MAX_VIEWS];
+    if ((int)threadIdx.x < g1 - g0) {
+        const DevView& G = tab.v[g0 + threadIdx.x];
+        s_view[threadIdx.x] = ResolveView{G.vert, G.color, G.z, G.w, G.tri_shift, G.color_scale, 0};
+    }
+    __syncthreads();
     const size_t npo = (size_t)T.wo * T.ho;
     const size_t po = inside ? (size_t)y * T.wo + x : 0;
     BlendAcc a = {0.f, 0.f, 0.f, 0.f};
@@ -51,11 +76,11 @@ __global__ void __launch_bounds__(TILE_W * TILE_H) resolve_kernel(const __grid_c
             adepth = tab.aux.acc_depth[po];
             avalid = tab.aux.acc_valid[po];
         }
-        unsigned long long key = __ldg(tab.v[g0].z + po);
+        unsigned long long key = __ldg(s_view[0].z + po);
         for (int v = g0; v < g1; ++v) {
             const unsigned long long cur = key;
-            if (v + 1 < g1) key = __ldg(tab.v[v + 1].z + po);
-            const Fragment f = resolve_fragment(tab.v[v], cur, x, y, T.precision);
+            if (v + 1 < g1) key = __ldg(s_view[v + 1 - g0].z + po);
+            const Fragment f = resolve_fragment(s_view[v - g0], cur, x, y, T.precision);
             const float qv = __fdiv_rn(f.validity, f.depth);
             if (Extras && tab.ms.on) tab.ms.view[(size_t)v * npo + po] = make_float4(f.col.x, f.col.y, f.col.z, qv);
             if (aux) {
