@@ -214,10 +214,15 @@ __device__ __forceinline__ bool tri_range(float4 A, float4 B, float4 C, int wo, 
 
 // Candidate x range of row y for a large triangle.  Each edge test
 // n_k = a_k*tx + b_k*ty + c_k >= -1e-6*den (n_3 = den - n_1 - n_2) bounds tx
-// on one side; the bound is widened by 16 ulp of its terms plus 1e-3 and
-// then by one pixel, and an edge whose bound is not reliable to half a pixel
-// (nearly horizontal edges) is not used.  Every pixel of the span is still
-// tested exactly, so the span only has to contain the covered pixels.
+// on one side; the bound is widened by 16 ulp of its terms plus 1e-3, and an
+// edge whose bound is not reliable to half a pixel (nearly horizontal edges)
+// is not used.  Turned into pixels it is widened by another 0.01, which covers
+// the rounding of cx - 0.5 + bound (at most 3 roundings of values below 2^16,
+// under 0.004 each where the pixel lies in an image at most 32768 wide).
+// Every pixel of the span is still tested exactly, so the span only has to
+// contain the covered pixels.  (Stretched triangles are thin: widened by a
+// whole pixel on either side, a row of one covered pixel had three
+// candidates or more, and the kernel took twice as long.)
 __device__ __forceinline__ void row_span(const TriSetup& s, float cx, float cy, int y, int& xl, int& xr) {
     const float eps = 1e-6f, u = 5.9604645e-8f;
     const float ty = __fsub_rn(__fadd_rn((float)y, 0.5f), cy);
@@ -244,8 +249,8 @@ __device__ __forceinline__ void row_span(const TriSetup& s, float cx, float cy, 
     }
     xl = s.x0;
     xr = s.x1;
-    if (lo > -INFINITY) xl = max(xl, (int)fmaxf(-1.0e9f, floorf(cx - 0.5f + lo) - 1.f));
-    if (hi < INFINITY) xr = min(xr, (int)fminf(1.0e9f, ceilf(cx - 0.5f + hi) + 1.f));
+    if (lo > -INFINITY) xl = max(xl, (int)fmaxf(-1.0e9f, ceilf(cx - 0.5f + lo - 0.01f)));
+    if (hi < INFINITY) xr = min(xr, (int)fminf(1.0e9f, floorf(cx - 0.5f + hi + 0.01f)));
     if (empty) xr = xl - 1;
 }
 
