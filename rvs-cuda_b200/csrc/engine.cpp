@@ -426,7 +426,19 @@ float pixels_per_radian(const rvsb_camera& c) {
     return c.focal[0];
 }
 
-// Raster variant of a run that is neither pinned nor tuned.
+// Raster variant of a run that is neither pinned nor tuned.  An input pixel
+// spacing seen m times magnified in the raster gives triangles whose
+// candidate boxes hold about (m + 1)^2 pixels: at m = 1 one or two, and then
+// the few above 4 go to the list of large triangles; past m of about 1.1 the
+// threshold is 16, so that the ordinary triangles stay with their lanes: 2 x
+// 960x540 into 1920x1080 (m = 2) 158 us against 249 with 4, 8 views of 4 ERP
+// 4096x2048 inputs (m = 1.47) 2.06 ms against 2.75.  At m <= 1 a threshold of
+// 16 costs up to 6% (4 x 1920x1080 into 960x540 245 us against 232).  An
+// equirectangular output stretches its rows by 1 / cos(latitude), sqrt(2) at
+// the median row, which its m includes (4 x ERP 4096x2048 into the same: 1.67
+// ms against 1.81).  The largest m of the batch decides.  The unmagnified
+// classes (one view, one minified to m <= 0.6, a batch of 8 or more) share
+// their parameters; the rows per warp follow the launch's size (mesh.cu).
 constexpr int kMagnifiedVariant = 7;
 constexpr int kDefaultVariant = 4;
 constexpr int kMinifiedVariant = 2;

@@ -70,20 +70,27 @@ template <class Tabs>
 int launch_batch(const Tabs& tabs, const BatchShape& shape, cudaStream_t stream, cudaEvent_t* events = nullptr);
 
 // Raster variants the autotuner chooses from: quad rows per warp of the mesh
-// kernel and the candidate pixels above which a triangle goes to the list of
-// large ones.  Every variant gives identical results.
+// kernel (0: by the launch's size) and the candidate pixels above which a
+// triangle goes to the list of large ones.  Every variant gives identical
+// results.
 struct RasterVariant {
     int rows, small;
 };
 constexpr int NUM_RASTER_VARIANTS = 8;
 constexpr RasterVariant kRasterVariants[NUM_RASTER_VARIANTS] = {
-    {16, 4}, {16, 8}, {32, 4}, {32, 8}, {16, 8}, {8, 16}, {16, 64}, {16, 16},
+    {4, 4}, {0, 4}, {0, 4}, {8, 8}, {0, 4}, {16, 4}, {32, 16}, {0, 16},
 };
 constexpr bool rows_divide_tiles() {
     for (const RasterVariant& v : kRasterVariants)
-        if (WARP_TILE % v.rows != 0) return false;
+        if (v.rows != 0 && WARP_TILE % v.rows != 0) return false;
     return true;
 }
+constexpr bool small_has_kernel() {
+    for (const RasterVariant& v : kRasterVariants)
+        if (v.small != 4 && v.small != 8 && v.small != 16) return false;
+    return true;
+}
+static_assert(small_has_kernel(), "a threshold without an instantiation of the mesh kernel");
 static_assert(rows_divide_tiles(), "a warp's quad rows must lie in one row of culling tiles");
 
 // Shared memory of the multispectral row sums for outputs up to max_wo wide.

@@ -483,43 +483,107 @@ __device__ __forceinline__ unsigned long long frag_key(float d, float invq, uint
     return ((unsigned long long)hi << 32) | tri;
 }
 
-// One warp rasterises triangle (A, B, C), set up in s with its candidate box:
-// the candidate span of each row, one lane per row and 32 rows at a time,
-// then the spans' pixels flattened over the warp, 32 candidates per round
-// whatever the shape.
-__device__ __forceinline__ void raster_large(const TriSetup& s, float4 A, float4 B, float4 C, float invq,
-                                             uint32_t tri, unsigned long long* z, int wo, int lane) {
-    for (int yb = s.y0; yb <= s.y1; yb += 32) {
+// A triangle set up for the warp: its coefficients and candidate box, and what
+// a fragment's key needs.
+struct Large {
+    TriSetup s;
+    float cx, cy, za, zb, zc, invq;
+    uint32_t tri;
+    unsigned long long* z;
+};
+
+__device__ __forceinline__ void plot(const Large& t, int wo, int x, int y) {
+    float d;
+    if (test_pixel(t.s, t.cx, t.cy, t.za, t.zb, t.zc, x, y, d))
+        atomicMin(t.z + (size_t)y * wo + x, frag_key(d, t.invq, t.tri));
+}
+
+__device__ __forceinline__ int incl_sum(int v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    return v;
+}
+
+// Owner of item `c` of a flattened sequence: the number of lanes whose
+// inclusive prefix is at most c (binary search).
+__device__ __forceinline__ int owner_of(int incl, int c) {
+    int own = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const int probe = __shfl_sync(0xffffffffu, incl, own + step - 1);
+        if (probe <= c) own += step;
+    }
+    return own;
+}
+
+// The triangle set up by lane `k`.
+__device__ __forceinline__ Large from_lane(const Large& t, int k) {
+    Large r;
+    r.s.b1c1 = __shfl_sync(0xffffffffu, t.s.b1c1, k);
+    r.s.c0b0 = __shfl_sync(0xffffffffu, t.s.c0b0, k);
+    r.s.c1a1 = __shfl_sync(0xffffffffu, t.s.c1a1, k);
+    r.s.a0c0 = __shfl_sync(0xffffffffu, t.s.a0c0, k);
+    r.s.den = __shfl_sync(0xffffffffu, t.s.den, k);
+    r.s.rinv = __shfl_sync(0xffffffffu, t.s.rinv, k);
+    r.s.x0 = __shfl_sync(0xffffffffu, t.s.x0, k);
+    r.s.x1 = __shfl_sync(0xffffffffu, t.s.x1, k);
+    r.s.y0 = __shfl_sync(0xffffffffu, t.s.y0, k);
+    r.s.y1 = __shfl_sync(0xffffffffu, t.s.y1, k);
+    r.cx = __shfl_sync(0xffffffffu, t.cx, k);
+    r.cy = __shfl_sync(0xffffffffu, t.cy, k);
+    r.za = __shfl_sync(0xffffffffu, t.za, k);
+    r.zb = __shfl_sync(0xffffffffu, t.zb, k);
+    r.zc = __shfl_sync(0xffffffffu, t.zc, k);
+    r.invq = __shfl_sync(0xffffffffu, t.invq, k);
+    r.tri = __shfl_sync(0xffffffffu, t.tri, k);
+    r.z = reinterpret_cast<unsigned long long*>(
+        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(t.z), k));
+    return r;
+}
+
+// One warp rasterises a triangle: the candidate span of each row, one lane
+// per row and 32 rows at a time, then the spans' pixels flattened over the
+// warp, 32 candidates per round whatever the shape.
+__device__ __forceinline__ void raster_large(const Large& t, int wo, int lane) {
+    for (int yb = t.s.y0; yb <= t.s.y1; yb += 32) {
         const int y = yb + lane;
         int xl = 0, xr = -1;
-        if (y <= s.y1) row_span(s, C.x, C.y, y, xl, xr);
+        if (y <= t.s.y1) row_span(t.s, t.cx, t.cy, y, xl, xr);
         const int len = max(0, xr - xl + 1);
-        int incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
+        const int incl = incl_sum(len, lane);
         const int excl = incl - len;
         const int total = __shfl_sync(0xffffffffu, incl, 31);
         for (int base = 0; base < total; base += 32) {
             const int c = base + lane;
-            // Row of candidate c: the number of rows whose spans end at
-            // or before c (binary search over the inclusive prefix).
-            int row = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int probe = __shfl_sync(0xffffffffu, incl, row + step - 1);
-                if (probe <= c) row += step;
-            }
+            const int row = owner_of(incl, c);
             const int rxl = __shfl_sync(0xffffffffu, xl, row);
             const int rex = __shfl_sync(0xffffffffu, excl, row);
-            if (c >= total) continue;
-            const int x = rxl + (c - rex), yy = yb + row;
-            float d;
-            if (test_pixel(s, C.x, C.y, A.z, B.z, C.z, x, yy, d))
-                atomicMin(z + (size_t)yy * wo + x, frag_key(d, invq, tri));
+            if (c < total) plot(t, wo, rxl + (c - rex), yb + row);
         }
+    }
+}
+
+// The warp's triangles (one per lane that is `on`) with their boxes flattened
+// together, 32 candidates per round.
+constexpr int kMediumPixels = 64;
+__device__ __forceinline__ void raster_medium(const Large& t, bool on, int wo, int lane) {
+    const int bw = t.s.x1 - t.s.x0 + 1;
+    const int count = on ? bw * (t.s.y1 - t.s.y0 + 1) : 0;
+    const int incl = incl_sum(count, lane);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int base = 0; base < total; base += 32) {
+        const int c = base + lane;
+        const int own = owner_of(incl, c) & 31;
+        const Large r = from_lane(t, own);
+        const int k = c - __shfl_sync(0xffffffffu, incl - count, own), w = __shfl_sync(0xffffffffu, bw, own);
+        if (c >= total) continue;
+        // k and w are at most 64: (k + 0.5) / w is at least 1/128 from an
+        // integer, so the fast quotient truncates to the exact row.
+        const int dy = (int)__fdividef((float)k + 0.5f, (float)w);
+        plot(r, wo, r.s.x0 + (k - dy * w), r.s.y0 + dy);
     }
 }
 
@@ -533,13 +597,57 @@ __device__ __forceinline__ void load_triangle(const DevView& V, uint32_t tri, fl
     C = __ldg(V.vert + (size_t)cy * V.w + cx);
 }
 
-// Grid (CTAs, slots), LARGE_THREADS threads: every warp takes entries of the
-// slot's list in turn.  When the list overflowed (more large triangles than
-// it holds), the warps instead go over all quads of the group's views and
+// Triangle `tri` of view V set up for rasterisation.  False when nothing of it
+// can be covered.  Its candidate box is (x0, y0) .. (x1, y1) where `box` says
+// so, else computed (the whole triangle).
+__device__ __forceinline__ bool set_up(const DevView& V, const DevTarget& T, uint32_t tri, bool box, Large& t) {
+    float4 A, B, C;
+    load_triangle(V, tri, A, B, C);
+    const int x0 = t.s.x0, x1 = t.s.x1, y0 = t.s.y0, y1 = t.s.y1;
+    if (!tri_coef(A, B, C, t.s)) return false;
+    if (box) {
+        t.s.x0 = x0; t.s.x1 = x1; t.s.y0 = y0; t.s.y1 = y1;
+    } else if (!tri_range(A, B, C, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, t.s)) {
+        return false;
+    }
+    t.s.rinv = rcp_approx(t.s.den);
+    t.cx = C.x; t.cy = C.y;
+    t.za = A.z; t.zb = B.z; t.zc = C.z;
+    t.invq = key_invq(A, B, C, T.precision);
+    t.tri = tri;
+    t.z = V.z;
+    return true;
+}
+
+// Whether a list entry is of at most kMediumPixels candidates (its box known).
+__device__ __forceinline__ bool is_medium(uint4 q) {
+    return !(q.y & 256u) &&
+           ((q.z >> 16) - (q.z & 0xffffu) + 1u) * ((q.w >> 16) - (q.w & 0xffffu) + 1u) <= (uint32_t)kMediumPixels;
+}
+
+__device__ __forceinline__ bool set_up_entry(const SlotTable& tab, uint4 q, Large& t) {
+    t.s.x0 = (int)(q.z & 0xffffu);
+    t.s.x1 = (int)(q.z >> 16);
+    t.s.y0 = (int)(q.w & 0xffffu);
+    t.s.y1 = (int)(q.w >> 16);
+    return set_up(tab.v[q.y & 255u], tab.t, q.x, !(q.y & 256u), t);
+}
+
+// Grid (CTAs, slots), LARGE_THREADS threads, over the slot's list.  Medium
+// entries: a warp takes up to 32 consecutive ones (fewer when the list is
+// short, so that all warps have some), sets them up one per lane and
+// rasterises them together; 2 x 960x540 magnified twice with a threshold of 4
+// candidates lists nearly every triangle, 111 us against 995 us with a warp per
+// entry.  The others go one by one to the warps, dealt out in turn: they are
+// few and differ in size, and neighbours in the list are alike (a warp that
+// took 32 in a row kept the kernel waiting: 590 instead of 178 us, ERP to ERP).
+//
+// When the list overflowed (more large triangles than it holds), the warps
+// instead go over all quads of the group's views and
 // rasterise every triangle; those the mesh kernel has done already only
 // repeat keys that are there (atomicMin).
 template <class Tabs>
-__global__ void __launch_bounds__(LARGE_THREADS) large_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
+__global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.y);
     const DevTarget& T = tab.t;
@@ -548,23 +656,31 @@ __global__ void __launch_bounds__(LARGE_THREADS) large_kernel(const __grid_const
     const int lane = threadIdx.x & 31;
     const int wid = blockIdx.x * (LARGE_THREADS / 32) + (threadIdx.x >> 5), nw = gridDim.x * (LARGE_THREADS / 32);
     if (n <= tab.b.large_capacity) {
-        for (int e = wid; e < n; e += nw) {
-            const uint4 q = __ldg(tab.b.large + e);
-            const DevView& V = tab.v[q.y & 255u];
-            float4 A, B, C;
-            load_triangle(V, q.x, A, B, C);
-            TriSetup s;
-            if (!tri_coef(A, B, C, s)) continue;
-            if (q.y & 256u) {
-                if (!tri_range(A, B, C, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, s)) continue;
-            } else {
-                s.x0 = (int)(q.z & 0xffffu);
-                s.x1 = (int)(q.z >> 16);
-                s.y0 = (int)(q.w & 0xffffu);
-                s.y1 = (int)(q.w >> 16);
+        const uint4* list = tab.b.large;
+        for (int base = 0; base < n; base += 32 * nw) {
+            // Lane k looks at the warp's k-th entry of the round.
+            const int e = base + lane * nw + wid;
+            uint4 q = make_uint4(0u, 0u, 0u, 0u);
+            if (e < n) q = __ldg(list + e);
+            for (unsigned m = __ballot_sync(0xffffffffu, e < n && !is_medium(q)); m; m &= m - 1) {
+                const int k = __ffs(m) - 1;
+                Large t;
+                if (set_up_entry(tab,
+                                 make_uint4(__shfl_sync(0xffffffffu, q.x, k), __shfl_sync(0xffffffffu, q.y, k),
+                                            __shfl_sync(0xffffffffu, q.z, k), __shfl_sync(0xffffffffu, q.w, k)),
+                                 t))
+                    raster_large(t, T.wo, lane);
             }
-            s.rinv = rcp_approx(s.den);
-            raster_large(s, A, B, C, key_invq(A, B, C, T.precision), q.x, V.z, T.wo, lane);
+        }
+        const int per = min(32, (n + nw - 1) / nw);
+        for (int e0 = wid * per; e0 < n; e0 += nw * per) {
+            Large t = {};
+            bool on = lane < per && e0 + lane < n;
+            if (on) {
+                const uint4 q = __ldg(list + e0 + lane);
+                on = is_medium(q) && set_up_entry(tab, q, t);
+            }
+            raster_medium(t, on, T.wo, lane);
         }
         return;
     }
@@ -577,26 +693,20 @@ __global__ void __launch_bounds__(LARGE_THREADS) large_kernel(const __grid_const
             if (T.cull && V.erp_cone && tile_culled(V, T, j0 / WARP_TILE, i / WARP_TILE)) continue;
             for (int t = 0; t < (wrap ? 4 : 2); ++t) {
                 const uint32_t tri = ((((uint32_t)i << (V.tri_shift - 2)) | (uint32_t)j) << 2) | (uint32_t)t;
-                float4 A, B, C;
-                TriSetup s;
+                Large r = {};
                 bool on = j < V.w - 1 && (t < 2 || j == 0);
                 if (on) {
+                    // Emission tests of transform.cpp:161-167.
                     const float4 v01 = __ldg(V.vert + (size_t)i * V.w + j + 1);
                     const float4 v10 = __ldg(V.vert + (size_t)(i + 1) * V.w + j);
-                    load_triangle(V, tri, A, B, C);
+                    const float4 a = __ldg(V.vert + (size_t)(i + (t & 1)) * V.w + j + (t & 1));
                     on = v01.z > 0.f && v10.z > 0.f && v01.x > 0.f && v10.x > 0.f &&
-                         (t >= 2 || (A.z > 0.f && A.x > 0.f)) && tri_coef(A, B, C, s) &&
-                         tri_range(A, B, C, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, s);
+                         (t >= 2 || (a.z > 0.f && a.x > 0.f)) && set_up(V, T, tri, false, r);
                 }
-                for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
-                    const uint32_t k = __shfl_sync(0xffffffffu, tri, __ffs(m) - 1);
-                    float4 a, b, c;
-                    TriSetup r;
-                    load_triangle(V, k, a, b, c);
-                    if (!tri_coef(a, b, c, r) || !tri_range(a, b, c, T.wo, T.ho, 0, T.wo - 1, 0, T.ho - 1, r)) continue;
-                    r.rinv = rcp_approx(r.den);
-                    raster_large(r, a, b, c, key_invq(a, b, c, T.precision), k, V.z, T.wo, lane);
-                }
+                const bool medium = on && (r.s.x1 - r.s.x0 + 1) * (r.s.y1 - r.s.y0 + 1) <= kMediumPixels;
+                raster_medium(r, medium, T.wo, lane);
+                for (unsigned m = __ballot_sync(0xffffffffu, on && !medium); m; m &= m - 1)
+                    raster_large(from_lane(r, __ffs(m) - 1), T.wo, lane);
             }
         }
     }
@@ -620,17 +730,31 @@ __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Tabs
 
 }  // namespace
 
+// Quad rows per warp, by how many waves of warps (148 SMs x 32) 8 rows each
+// would make.  More rows warp fewer vertices twice (one row of 1 + 1 / rows),
+// fewer leave shorter warps at the end of the launch.  Below 2 waves 4 rows: 2
+// x 960x540 43 us the stage, 49 with 8, 61 with 16.  Below 40 waves 8: 4 x
+// 1920x1080 193 us (16 rows: 196), 4 x ERP 4096x2048 into ERP 1076 (16: 1121,
+// 32: 1156).  Above, where the end does not matter, 32: 8 poses of the 1080p
+// scene 160 us a view (8: 166), 8 views of the ERP scene 122 (16: 128, 8: 145;
+// a warp also decides there whether its rows are culled at all).
+static int rows_per_warp(const BatchShape& sh, int gv) {
+    const long long warps = (long long)sh.slots * gv * ((sh.max_w - 1 + STRIP - 1) / STRIP) * ((sh.max_h + 6) / 8);
+    const long long wave = 148 * 32;
+    return warps < 2 * wave ? 4 : warps < 40 * wave ? 8 : 32;
+}
+
 template <bool kErpOut, class Tabs>
 static void launch_mesh_kernel(const Tabs& tabs, const BatchShape& sh, int g0, int gv, cudaStream_t s) {
-    const RasterVariant& rv = kRasterVariants[sh.variant];
+    RasterVariant rv = kRasterVariants[sh.variant];
+    if (rv.rows == 0) rv.rows = rows_per_warp(sh, gv);
     const int strips = (sh.max_w - 1 + STRIP - 1) / STRIP + (kErpOut ? 1 : 0);  // and the seam's
     const dim3 grid((strips + MESH_WARPS - 1) / MESH_WARPS, (sh.max_h - 1 + rv.rows - 1) / rv.rows, sh.slots * gv);
     auto go = [&](auto kernel) { launch_dependent(kernel, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); };
     switch (rv.small) {
         case 4: go(mesh_kernel<4, kErpOut, Tabs>); break;
         case 8: go(mesh_kernel<8, kErpOut, Tabs>); break;
-        case 16: go(mesh_kernel<16, kErpOut, Tabs>); break;
-        default: go(mesh_kernel<64, kErpOut, Tabs>); break;
+        default: go(mesh_kernel<16, kErpOut, Tabs>); break;
     }
 }
 
