@@ -13,6 +13,7 @@
 #include <cstdint>
 
 #include "device_types.hpp"
+#include "erp_trig.cuh"
 
 namespace rvsb {
 namespace dev {
@@ -103,14 +104,8 @@ __device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T,
     }
     float u, v, z;
     if (kErpOut && T.proj == 1) {
-        double s2 = 0.0;
-        s2 = __dadd_rn(s2, __dmul_rn((double)y[0], (double)y[0]));
-        s2 = __dadd_rn(s2, __dmul_rn((double)y[1], (double)y[1]));
-        s2 = __dadd_rn(s2, __dmul_rn((double)y[2], (double)y[2]));
-        const float radius = (float)__dsqrt_rn(s2);
-        z = radius;
-        const float phi = (float)atan2((double)y[1], (double)y[0]);
-        const float theta = (float)asin((double)__fdiv_rn(y[2], radius));
+        float phi, theta;
+        erp_direction(y[0], y[1], y[2], z, phi, theta);
         u = __fadd_rn(T.u0, __fmul_rn(T.du_dphi, phi));
         v = __fadd_rn(T.v0, __fmul_rn(T.dv_dtheta, theta));
     } else {
