@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -168,7 +169,8 @@ BatchCore& single_core(rvsb_scene* sc) {
 // their colour is decoded into the scene and their depth read in place.
 rvsb_status synthesize_impl(rvsb_scene* sc, const rvsb_camera* virt, const rvsb_synth_params* params,
                             const rvsb_yuv420* out, const rvsb_debug_out* dbg_out, void* stream,
-                            const rvsb_view_planes* frame = nullptr, const rvsb_aux_out* aux = nullptr) {
+                            const rvsb_view_planes* frame = nullptr, const rvsb_aux_out* aux = nullptr,
+                            const std::function<void()>& before_resolve = {}) {
     if (!sc) return RVSB_E_ARG;
     rvsb_context* ctx = sc->ctx;
     HostRange range("rvsb: synthesize");
@@ -236,7 +238,7 @@ rvsb_status synthesize_impl(rvsb_scene* sc, const rvsb_camera* virt, const rvsb_
             r.dbg.blend_quality = dbg_out->blend_quality;
             r.dbg.inpaint_source = dbg_out->inpaint_source;
         }
-        const int launches = core.run(&r, 1, s);
+        const int launches = core.run(&r, 1, s, before_resolve);
         if (r.dbg.warped_uvz) {
             size_t off = 0;
             SlotWorkspace& ws = core.workspace(0);
@@ -293,10 +295,10 @@ rvsb_status rvsb_create(int device, size_t hbm_budget_bytes, rvsb_context** out)
 void rvsb_destroy(rvsb_context* ctx) {
     if (!ctx) return;
     if (ctx->host_scene) rvsb_scene_destroy(ctx->host_scene);
-    if (ctx->host_out) {
-        cudaSetDevice(ctx->device);
-        cudaFree(ctx->host_out);
-    }
+    cudaSetDevice(ctx->device);
+    if (ctx->host_out) cudaFree(ctx->host_out);
+    if (ctx->host_copy) cudaStreamDestroy(ctx->host_copy);
+    if (ctx->host_ready) cudaEventDestroy(ctx->host_ready);
     delete ctx;
 }
 
@@ -578,11 +580,10 @@ rvsb_status rvsb_synthesize_host(rvsb_context* ctx, const rvsb_camera* inputs, i
         if (st != RVSB_OK) return st;
         ctx->host_scene = sc;
     }
-    for (int v = 0; v < n_inputs; ++v) {
-        rvsb_status st = rvsb_scene_upload(sc, v, &host_planes[v], 0, stream);
-        if (st != RVSB_OK) return st;
-    }
     return guarded(ctx, [&]() -> rvsb_status {
+        for (int v = 0; v < n_inputs; ++v)
+            if (!host_planes[v].y || !host_planes[v].u || !host_planes[v].v || !host_planes[v].depth)
+                throw ArgError("null plane");
         if (!out_host->y || !out_host->u || !out_host->v) throw ArgError("null output planes");
         const size_t ny = (size_t)virt->width * virt->height * 2;
         const size_t nc = (size_t)(virt->width / 2) * (virt->height / 2) * 2;
@@ -604,9 +605,61 @@ rvsb_status rvsb_synthesize_host(rvsb_context* ctx, const rvsb_camera* inputs, i
         dev.y = reinterpret_cast<uint16_t*>(base);
         dev.u = reinterpret_cast<uint16_t*>(base + ny);
         dev.v = reinterpret_cast<uint16_t*>(base + ny + nc);
-        rvsb_status st = synthesize_impl(sc, virt, params, &dev, nullptr, stream);
-        if (st != RVSB_OK) return st;
+        // The depth planes go up first, on a stream of their own: the mesh
+        // kernels need nothing else of the inputs and run while the colour
+        // planes (three fifths of the bytes) are still on their way; each
+        // view's colour is decoded as it arrives.  4 x 1920x1080 (41.5 MB up):
+        // 1374 -> 1125 us a call, of which the link takes 870.
         cudaStream_t s = static_cast<cudaStream_t>(stream);
+        check(cudaSetDevice(ctx->device), "cudaSetDevice");
+        if (!ctx->host_copy) check(cudaStreamCreateWithFlags(&ctx->host_copy, cudaStreamNonBlocking), "cudaStreamCreate");
+        if (!ctx->host_ready)
+            check(cudaEventCreateWithFlags(&ctx->host_ready, cudaEventDisableTiming), "cudaEventCreate");
+        // `to` waits for what has been issued on `from` so far.
+        auto order = [&](cudaStream_t from, cudaStream_t to) {
+            check(cudaEventRecord(ctx->host_ready, from), "record upload");
+            check(cudaStreamWaitEvent(to, ctx->host_ready, 0), "wait for upload");
+        };
+        // Copies still reading the caller's planes when an error ends the call.
+        struct CopiesDone {
+            cudaStream_t s;
+            ~CopiesDone() { cudaStreamSynchronize(s); }
+        } copies_done{ctx->host_copy};
+        order(s, ctx->host_copy);
+        TileDepthJobs jobs{};
+        int n_erp = 0, ew = 0, eh = 0;
+        for (int v = 0; v < n_inputs; ++v) {
+            const rvsb_camera& c = sc->cams[v];
+            check(cudaMemcpyAsync(sc->plane(v, 3), host_planes[v].depth, plane_bytes(c, 3), cudaMemcpyHostToDevice,
+                                  ctx->host_copy),
+                  "upload planes");
+            sc->uploaded[v] = true;
+            if (c.projection != RVSB_PROJ_EQUIRECTANGULAR) continue;
+            jobs.v[n_erp++] = TileDepthJob{sc->plane(v, 3), sc->depth_lut[v]->as<float4>(),
+                                           sc->tile_depth[v]->as<float2>(), c.width, c.height};
+            ew = std::max(ew, c.width);
+            eh = std::max(eh, c.height);
+        }
+        order(ctx->host_copy, s);
+        if (n_erp > 0) {
+            launch_tile_depth(jobs, n_erp, ew, eh, s);
+            check(cudaPeekAtLastError(), "tile depth ranges");
+        }
+        auto colours = [&] {
+            for (int v = 0; v < n_inputs; ++v) {
+                const rvsb_camera& c = sc->cams[v];
+                const void* src[3] = {host_planes[v].y, host_planes[v].u, host_planes[v].v};
+                CopyPart parts[3];
+                for (int k = 0; k < 3; ++k) parts[k] = {sc->plane(v, k), src[k], plane_bytes(c, k)};
+                copy_planes(parts, 3, cudaMemcpyHostToDevice, ctx->host_copy, "upload planes");
+                order(ctx->host_copy, s);
+                launch_decode_color(sc->plane(v, 0), sc->plane(v, 1), sc->plane(v, 2), c.width, c.height,
+                                    sc->color[v]->as<uint64_t>(), s);
+                check(cudaPeekAtLastError(), "decode colour");
+            }
+        };
+        rvsb_status st = synthesize_impl(sc, virt, params, &dev, nullptr, stream, nullptr, nullptr, colours);
+        if (st != RVSB_OK) return st;
         download_yuv(out_host, dev, ny, nc, s);
         check(cudaStreamSynchronize(s), "synchronize");
         return RVSB_OK;

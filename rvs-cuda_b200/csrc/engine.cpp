@@ -369,13 +369,14 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
     return sh;
 }
 
-int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaStream_t s) {
+int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaStream_t s,
+                              const std::function<void()>& before_resolve) {
     const BatchShape sh = shape_of(reqs, n, variant);
-    if (n == 1 && !use_graphs_) {
+    if (n == 1 && (!use_graphs_ || before_resolve)) {
         // A single synthesis: the table travels as a kernel parameter.
         TableParam tp;
         fill(tp.t, 0, reqs[0], sh);
-        const int launches = launch_batch(tp, sh, s, profiling_ ? events_ : nullptr);
+        const int launches = launch_batch(tp, sh, s, profiling_ ? events_ : nullptr, before_resolve);
         if (launches < 0) check(cudaGetLastError(), "kernel launch");
         return launches;
     }
@@ -507,7 +508,7 @@ int BatchCore::tune(const SlotRequest* reqs, int n, cudaStream_t s) {
     return best;
 }
 
-int BatchCore::run(const SlotRequest* reqs, int n, cudaStream_t s) {
+int BatchCore::run(const SlotRequest* reqs, int n, cudaStream_t s, const std::function<void()>& before_resolve) {
     HostRange range("rvsb: batch (tables, launches)");
     if (n <= 0 || n > slots_) throw ArgError("batch of " + std::to_string(n) + " requests for " +
                                              std::to_string(slots_) + " slots");
@@ -547,7 +548,7 @@ int BatchCore::run(const SlotRequest* reqs, int n, cudaStream_t s) {
         if (it == tuned_.end()) it = tuned_.emplace(sig, tune(reqs, n, s)).first;
         variant = it->second;
     }
-    const int launches = launch_variant(reqs, n, variant, s);
+    const int launches = launch_variant(reqs, n, variant, s, before_resolve);
     profiled_ = profiling_;
     last_launches_ = launches;
     last_variant_ = variant;

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -51,6 +52,8 @@ struct rvsb_context {
     rvsb_scene* host_scene = nullptr;  // scene reused by rvsb_synthesize_host
     void* host_out = nullptr;          // device output staging of rvsb_synthesize_host
     size_t host_out_bytes = 0;
+    cudaStream_t host_copy = nullptr;  // uploads of rvsb_synthesize_host
+    cudaEvent_t host_ready = nullptr;  // orders them with the caller's stream
 };
 
 namespace rvsb {
@@ -137,7 +140,9 @@ public:
 
     // Sizes the slot workspaces for the requests, fills and uploads their
     // tables and issues the batch on `stream`.  Returns the kernel launches.
-    int run(const SlotRequest* reqs, int n, cudaStream_t stream);
+    // `before_resolve` (optional) runs between the mesh kernels, which read
+    // the inputs' depth alone, and the resolve, which reads their colour.
+    int run(const SlotRequest* reqs, int n, cudaStream_t stream, const std::function<void()>& before_resolve = {});
 
     void set_graphs(bool on) { use_graphs_ = on; }
     // Time every raster variant on the first batch of each new shape and
@@ -155,7 +160,8 @@ public:
 private:
     void fill(SlotTable& t, int k, const SlotRequest& r, const BatchShape& sh);
     BatchShape shape_of(const SlotRequest* reqs, int n, int variant) const;
-    int launch_variant(const SlotRequest* reqs, int n, int variant, cudaStream_t s);
+    int launch_variant(const SlotRequest* reqs, int n, int variant, cudaStream_t s,
+                       const std::function<void()>& before_resolve = {});
     int tune(const SlotRequest* reqs, int n, cudaStream_t s);
 
     rvsb_context* ctx_;

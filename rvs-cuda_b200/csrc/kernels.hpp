@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <cuda_runtime.h>
 
 #include "device_types.hpp"
@@ -64,10 +65,12 @@ void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
 
 // Issues one batch of syntheses on `stream`; returns the number of kernel
 // launches, or -1 on a launch error (cudaGetLastError holds the cause).
-// `events` (optional) holds 2 * NUM_STAGES events recorded around the stages.
+// `events` (optional) holds 2 * NUM_STAGES events recorded around the stages;
+// `before_resolve` (optional) is called before the first resolve is launched.
 constexpr int NUM_STAGES = 5;
 template <class Tabs>
-int launch_batch(const Tabs& tabs, const BatchShape& shape, cudaStream_t stream, cudaEvent_t* events = nullptr);
+int launch_batch(const Tabs& tabs, const BatchShape& shape, cudaStream_t stream, cudaEvent_t* events = nullptr,
+                 const std::function<void()>& before_resolve = {});
 
 // Raster variants the autotuner chooses from: quad rows per warp of the mesh
 // kernel (0: by the launch's size) and the candidate pixels above which a

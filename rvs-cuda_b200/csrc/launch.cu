@@ -34,7 +34,8 @@ __global__ void slot_init_kernel(const __grid_constant__ Tabs tabs) {
 }  // namespace
 
 template <class Tabs>
-int launch_batch(const Tabs& tabs, const BatchShape& sh, cudaStream_t s, cudaEvent_t* ev) {
+int launch_batch(const Tabs& tabs, const BatchShape& sh, cudaStream_t s, cudaEvent_t* ev,
+                 const std::function<void()>& before_resolve) {
     auto mark = [&](int k) {
         if (ev) cudaEventRecord(ev[k], s);
     };
@@ -44,6 +45,7 @@ int launch_batch(const Tabs& tabs, const BatchShape& sh, cudaStream_t s, cudaEve
     for (int g0 = 0; g0 < sh.max_views; g0 += sh.vg) {
         launches += launch_mesh(tabs, sh, g0, s, g0 == 0 ? ev : nullptr);
         if (g0 == 0) mark(4);
+        if (g0 == 0 && before_resolve) before_resolve();
         launch_resolve(tabs, sh, g0, s);
         ++launches;
     }
@@ -59,7 +61,9 @@ int launch_batch(const Tabs& tabs, const BatchShape& sh, cudaStream_t s, cudaEve
     return launches + (sh.aux ? 1 : 0) + (sh.rescale ? 1 : 0);
 }
 
-template int launch_batch<TableParam>(const TableParam&, const BatchShape&, cudaStream_t, cudaEvent_t*);
-template int launch_batch<TablePtr>(const TablePtr&, const BatchShape&, cudaStream_t, cudaEvent_t*);
+template int launch_batch<TableParam>(const TableParam&, const BatchShape&, cudaStream_t, cudaEvent_t*,
+                                      const std::function<void()>&);
+template int launch_batch<TablePtr>(const TablePtr&, const BatchShape&, cudaStream_t, cudaEvent_t*,
+                                    const std::function<void()>&);
 
 }  // namespace rvsb
