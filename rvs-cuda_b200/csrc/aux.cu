@@ -2,7 +2,7 @@
 // inpainting: the validity mask (View::get_validity_mask, View.cpp:206-211),
 // the masked colour (colour set to 0.5 where masked, then write_color), the
 // blended depth and the masked depth (write_maskedDepth,
-// image_writing.cpp:237-268).  One thread per 2x2 output block.
+// image_writing.cpp:237-268).
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -58,37 +58,40 @@ __device__ __forceinline__ int nearest_src(int d, int out, int raster) {
     return min((int)floor(__dmul_rn((double)d, ifx)), raster - 1);
 }
 
-// One thread per 2x2 block of the output (the virtual camera's size).  At
-// Precision != 1 the validity mask and the depth are computed at the raster
-// size and resized to the output (Pipeline.cpp:303-333): the mask with
-// INTER_NEAREST, the depth with INTER_LINEAR; the masked colour is not
-// produced there (the host refuses it).
+constexpr int AUX_W = 32, AUX_H = 8;
+
+// One thread per pixel of the output (the virtual camera's size, its sides
+// even), a warp 16 x 2 of them: the lanes of a chroma block exchange its
+// samples.  At Precision != 1 the validity mask and the depth are computed at
+// the raster size and resized to the output (Pipeline.cpp:303-333): the mask
+// with INTER_NEAREST, the depth with INTER_LINEAR; the masked colour is not
+// produced there (the host refuses it).  A thread per 2x2 block left too few
+// threads to cover the divisions' and loads' latency: 13.7 us on a 1278x718
+// output, the whole call 172 us, 169 so.
 template <class Tabs>
-__global__ void aux_kernel(const __grid_constant__ Tabs tabs) {
+__global__ void __launch_bounds__(AUX_W * AUX_H) aux_kernel(const __grid_constant__ Tabs tabs) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z);
     const AuxPtrs& A = tab.aux;
     if (!A.on) return;
     const DevTarget& T = tab.t;
     const int ow = T.rescale ? T.out_w : T.wo, oh = T.rescale ? T.out_h : T.ho;
-    const int bx = blockIdx.x * blockDim.x + threadIdx.x, by = blockIdx.y;
-    const int x0 = 2 * bx, y0 = 2 * by;
-    if (x0 >= ow || y0 >= oh) return;
-    const uint32_t grey = quantize(0.5f, T.max_val);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * AUX_W + (warp & 1) * 16 + (lane & 15);
+    const int y = blockIdx.y * AUX_H + (warp >> 1) * 2 + (lane >> 4);
+    const bool inside = x < ow && y < oh;
     uint32_t su = 0, sv = 0;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        const int x = x0 + (p & 1), y = y0 + (p >> 1);
+    if (inside) {
         const size_t o = (size_t)y * ow + x;
         const size_t ov = T.rescale ? (size_t)nearest_src(y, oh, T.ho) * T.wo + nearest_src(x, ow, T.wo) : o;
         const bool masked = !(A.acc_valid[ov] > A.threshold);
         if (A.mask) A.mask[o] = masked ? 255 : 0;
         if (A.masked_y) {
+            const uint32_t grey = quantize(0.5f, T.max_val);
             const uint64_t c = tab.b.codes[o];
-            const uint32_t yy = masked ? grey : (uint32_t)(c & 0xffff);
-            su += masked ? grey : (uint32_t)((c >> 16) & 0xffff);
-            sv += masked ? grey : (uint32_t)((c >> 32) & 0xffff);
-            A.masked_y[o] = (uint16_t)yy;
+            su = masked ? grey : (uint32_t)((c >> 16) & 0xffff);
+            sv = masked ? grey : (uint32_t)((c >> 32) & 0xffff);
+            A.masked_y[o] = (uint16_t)(masked ? grey : (uint32_t)(c & 0xffff));
         }
         if (A.depth || A.masked_depth) {
             const float dep = T.rescale ? resized_depth(T, A.acc_depth, x, y) : A.acc_depth[o];
@@ -97,9 +100,15 @@ __global__ void aux_kernel(const __grid_constant__ Tabs tabs) {
         }
     }
     if (A.masked_y) {
-        const size_t co = (size_t)by * (T.wo / 2) + bx;
-        A.masked_u[co] = quarter_round(su, T.chroma_ties_up);
-        A.masked_v[co] = quarter_round(sv, T.chroma_ties_up);
+        su += __shfl_xor_sync(0xffffffffu, su, 1);
+        sv += __shfl_xor_sync(0xffffffffu, sv, 1);
+        su += __shfl_xor_sync(0xffffffffu, su, 16);
+        sv += __shfl_xor_sync(0xffffffffu, sv, 16);
+        if (inside && !(lane & 17)) {
+            const size_t co = (size_t)(y / 2) * (T.wo / 2) + x / 2;
+            A.masked_u[co] = quarter_round(su, T.chroma_ties_up);
+            A.masked_v[co] = quarter_round(sv, T.chroma_ties_up);
+        }
     }
 }
 
@@ -107,10 +116,11 @@ __global__ void aux_kernel(const __grid_constant__ Tabs tabs) {
 
 template <class Tabs>
 void launch_aux(const Tabs& tabs, const BatchShape& sh, cudaStream_t s) {
-    // Output blocks: the raster size, or the output size where a slot
+    // Output size: the raster size, or the output size where a slot
     // rasterises at Precision != 1.
     const int w = std::max(sh.max_wo, sh.max_out_w), h = std::max(sh.max_ho, sh.max_out_h);
-    launch_dependent(aux_kernel<Tabs>, dim3((w / 2 + 127) / 128, h / 2, sh.slots), dim3(128), 0, s, tabs);
+    launch_dependent(aux_kernel<Tabs>, dim3((w + AUX_W - 1) / AUX_W, (h + AUX_H - 1) / AUX_H, sh.slots),
+                     dim3(AUX_W * AUX_H), 0, s, tabs);
 }
 
 template void launch_aux<TableParam>(const TableParam&, const BatchShape&, cudaStream_t);

@@ -120,7 +120,8 @@ struct AuxPtrs {
 // the masked box mean of each view's luma, and the blend kernel the two
 // frequency bands' blends.  Per view, npix = Wo*Ho entries each.
 struct MsPtrs {
-    float4* view;       // (Y, U, V, quality) per view and pixel
+    float2* yq;         // (Y, quality) per view and pixel: all the blur reads
+    float2* uv;         // (U, V) per view and pixel
     double* hsum;       // row-window sums of masked luma
     int* hcnt;          // row-window counts of masked pixels
     float* blur;        // blurred luma (0 outside the mask)

@@ -292,7 +292,8 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
         D.blend_exp_int = exp_int(p.low_freq_factor);
         D.blend_max = p.low_freq_factor < 0.f ? 1 : 0;
         MsPtrs& M = T.ms;
-        M.view = ws.ms_view.as<float4>();
+        M.yq = ws.ms_view.as<float2>();
+        M.uv = M.yq + (size_t)n * npix;
         M.hsum = ws.ms_hsum.as<double>();
         M.hcnt = ws.ms_hcnt.as<int>();
         M.blur = ws.ms_blur.as<float>();

@@ -217,7 +217,7 @@ template <class Src, bool PRE>
 __global__ void __launch_bounds__(32 * COL_WARPS) inpaint_cols0_kernel(const __grid_constant__ Src src) {
     grid_dep_wait();
     const InpaintImage im = src();
-    if (im.st->n_holes == 0) return;
+    if (PRE && im.st->n_holes == 0) return;
     __shared__ unsigned long long s_total[COL_WARPS][32], s_carry[COL_WARPS][32];
     const int G = group_count(im.ho), g = blockIdx.y, w = blockIdx.x;
     if (g >= G || w >= im.words) return;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) inpaint_rows1_kernel(const __g
     grid_dep_wait();
     const InpaintImage im = src();
     const int y = blockIdx.x;
-    if (y >= im.ho || im.st->n_holes == 0) return;
+    if (y >= im.ho) return;
     __shared__ unsigned long long s_min[MAX_WORDS + 1];
     __shared__ uint32_t s_own[MAX_WORDS + 1], s_up[MAX_WORDS];  // s_own[0]: left of the row
     __shared__ uint16_t s_list[MAX_WORDS];
@@ -426,7 +426,6 @@ template <class Src>
 __global__ void __launch_bounds__(32 * COL_WARPS) inpaint_cols1_kernel(const __grid_constant__ Src src) {
     grid_dep_wait();
     const InpaintImage im = src();
-    if (im.st->n_holes == 0) return;
     __shared__ unsigned long long s_c[COL_WARPS][32], s_o[COL_WARPS][32], s_cc[COL_WARPS][32], s_co[COL_WARPS][32];
     __shared__ uint64_t s_choice[GROUP][32];
     __shared__ uint32_t s_own[GROUP];

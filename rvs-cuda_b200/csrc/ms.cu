@@ -18,9 +18,9 @@ namespace {
 
 using namespace dev;
 
-constexpr int MS_THREADS = 256;
+constexpr int MS_THREADS = 512;
 constexpr int MS_WARPS = MS_THREADS / 32;
-constexpr int MS_CHUNKS = 8;   // 32-column chunks a warp holds at once
+constexpr int MS_CHUNKS = 4;   // 32-column chunks a warp holds at once
 constexpr int MS_COLS = 128;   // columns per CTA of the column windows
 constexpr int MS_ROWS = 64;    // rows a thread of it slides over
 constexpr int MS_BATCH = 8;    // of them loaded together
@@ -29,10 +29,12 @@ constexpr int MS_BATCH = 8;    // of them loaded together
 // exclusive prefix (double sums, integer counts) is built in shared memory:
 // each warp scans MS_CHUNKS chunks of 32 columns, loaded together and
 // coalesced, the warps' totals are added, and wide rows take several rounds.
-// (With a run of consecutive columns per thread, read twice, 16 bytes every
-// 128, the kernel took 162 us on 4 views of 1920x1080.)
+// Bound by latency between its barriers: 54 us on 4 views of 1920x1080 (66 MB
+// in, 100 out) with four 512-thread CTAs per SM, 60 with three, 62 with four
+// of 256 threads and twice the chunks; a run of consecutive columns per
+// thread, read twice, 16 bytes every 128, took 162.
 template <class Tabs>
-__global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_constant__ Tabs tabs) {
+__global__ void __launch_bounds__(MS_THREADS, 4) ms_rows_kernel(const __grid_constant__ Tabs tabs) {
     grid_dep_wait();
     extern __shared__ __align__(16) unsigned char s_raw[];
     const SlotTable& tab = tabs.at(blockIdx.z);
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_consta
     __shared__ double s_wsum[MS_WARPS];
     __shared__ int s_wcnt[MS_WARPS];
     const size_t npo = (size_t)T.wo * T.ho;
-    const float4* row = M.view + (size_t)v * npo + (size_t)y * w;
+    const float2* row = M.yq + (size_t)v * npo + (size_t)y * w;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double base = 0.0;
     int cbase = 0;
@@ -62,9 +64,9 @@ __global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_consta
 #pragma unroll
         for (int k = 0; k < MS_CHUNKS; ++k) {
             const int x = x0 + 32 * k;
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 c = make_float2(0.f, 0.f);
             if (x < w) c = row[x];
-            const bool in = c.w > 0.f && isfinite(c.x);
+            const bool in = c.y > 0.f && isfinite(c.x);
             mask[k] = __ballot_sync(0xffffffffu, in);
             s[k] = in ? (double)c.x : 0.0;
         }
@@ -128,11 +130,12 @@ __global__ void __launch_bounds__(MS_THREADS) ms_rows_kernel(const __grid_consta
 // 54 that reads each row sum 3.7 times instead of twice, but runs 17 times as
 // many threads, and the loads of MS_BATCH rows are in flight together: 54 us
 // on 4 views of 1920x1080 against 827 us with one thread per whole column
-// (60 CTAs of 128 threads on 148 SMs); 32 and 128 rows: 64 and 62 us.
+// (60 CTAs of 128 threads on 148 SMs); 32 and 128 rows: 64 and 62 us, 4 rows
+// in flight and 12 CTAs per SM 79.
 // Writes the blurred luma.
 // Grid (ceil(max_wo / MS_COLS) * segments, views, slots).
 template <class Tabs>
-__global__ void __launch_bounds__(MS_COLS) ms_cols_kernel(const __grid_constant__ Tabs tabs, int segments) {
+__global__ void __launch_bounds__(MS_COLS, 7) ms_cols_kernel(const __grid_constant__ Tabs tabs, int segments) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z);
     const MsPtrs& M = tab.ms;
@@ -180,14 +183,17 @@ __global__ void __launch_bounds__(MS_COLS) ms_cols_kernel(const __grid_constant_
 }
 
 constexpr int MS_TILE_W = 32, MS_TILE_H = 8;
+constexpr int MS_VIEWS = 4;
 
 // The two bands' blends per pixel, added: rewrites the colour part of the
 // codes (the holes stay the raster's) and the output samples of hole-free 2x2
 // blocks.  One thread per pixel, a warp 16 x 2 of them (the lanes of a chroma
-// block exchange its samples).  Grid (ceil(max_wo / 32), ceil(max_ho / 8),
-// slots).
+// block exchange its samples).  Bound by the latency of its loads: with
+// MS_VIEWS views' values loaded together 54 us on 4 views of 1920x1080 (180
+// MB, 28 us at the copy rate), one or two at a time 95.
+// Grid (ceil(max_wo / 32), ceil(max_ho / 8), slots).
 template <class Tabs>
-__global__ void __launch_bounds__(MS_TILE_W * MS_TILE_H) ms_blend_kernel(const __grid_constant__ Tabs tabs) {
+__global__ void __launch_bounds__(MS_TILE_W * MS_TILE_H, 6) ms_blend_kernel(const __grid_constant__ Tabs tabs) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z);
     const MsPtrs& M = tab.ms;
@@ -202,15 +208,29 @@ __global__ void __launch_bounds__(MS_TILE_W * MS_TILE_H) ms_blend_kernel(const _
     bool hole = false;
     if (inside) {
         BlendAcc lo = {0.f, 0.f, 0.f, 0.f}, hi = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-        for (int v = 0; v < T.n_views; ++v) {
-            const float4 c = M.view[(size_t)v * npo + o];
-            // 0 outside the mask of quality > 0
-            const float b = c.w > 0.f ? M.blur[(size_t)v * npo + o] : 0.f;
-            const float3 lowc = make_float3(b, c.y, c.z);
-            const float3 highc = make_float3(__fsub_rn(c.x, b), __fsub_rn(c.y, c.y), __fsub_rn(c.z, c.z));
-            blend_view(lo, v, lowc, c.w, M.low_exp, M.low_int, M.low_exp < 0.f);
-            blend_view(hi, v, highc, c.w, M.high_exp, M.high_int, M.high_exp < 0.f);
+        // The views' values MS_VIEWS at a time, before the blends that wait
+        // for them.
+        for (int v0 = 0; v0 < T.n_views; v0 += MS_VIEWS) {
+            float2 yq[MS_VIEWS], uv[MS_VIEWS];
+            float blur[MS_VIEWS];
+#pragma unroll
+            for (int k = 0; k < MS_VIEWS; ++k) {
+                const size_t q = (size_t)min(v0 + k, T.n_views - 1) * npo + o;
+                yq[k] = M.yq[q];
+                uv[k] = M.uv[q];
+                blur[k] = M.blur[q];
+            }
+#pragma unroll
+            for (int k = 0; k < MS_VIEWS; ++k) {
+                if (v0 + k >= T.n_views) break;
+                // 0 outside the mask of quality > 0
+                const float b = yq[k].y > 0.f ? blur[k] : 0.f;
+                const float3 lowc = make_float3(b, uv[k].x, uv[k].y);
+                const float3 highc = make_float3(__fsub_rn(yq[k].x, b), __fsub_rn(uv[k].x, uv[k].x),
+                                                 __fsub_rn(uv[k].y, uv[k].y));
+                blend_view(lo, v0 + k, lowc, yq[k].y, M.low_exp, M.low_int, M.low_exp < 0.f);
+                blend_view(hi, v0 + k, highc, yq[k].y, M.high_exp, M.high_int, M.high_exp < 0.f);
+            }
         }
         const float f0 = __fadd_rn(lo.c0, hi.c0), f1 = __fadd_rn(lo.c1, hi.c1), f2 = __fadd_rn(lo.c2, hi.c2);
         if (T.rescale) tab.b.pcolor[o] = make_float4(f0, f1, f2, 0.f);

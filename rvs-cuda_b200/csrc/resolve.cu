@@ -82,7 +82,10 @@ __global__ void __launch_bounds__(TILE_W * TILE_H, 5) resolve_kernel(const __gri
             if (v + 1 < g1) key = __ldg(s_view[v + 1 - g0].z + po);
             const Fragment f = resolve_fragment(s_view[v - g0], cur, x, y, T.precision);
             const float qv = __fdiv_rn(f.validity, f.depth);
-            if (Extras && tab.ms.on) tab.ms.view[(size_t)v * npo + po] = make_float4(f.col.x, f.col.y, f.col.z, qv);
+            if (Extras && tab.ms.on) {
+                tab.ms.yq[(size_t)v * npo + po] = make_float2(f.col.x, qv);
+                tab.ms.uv[(size_t)v * npo + po] = make_float2(f.col.y, f.col.z);
+            }
             if (aux) {
                 // BlendedView.cpp:205-208: the view's depth where its quality
                 // beats the accumulator's before this blend (view 0: its
