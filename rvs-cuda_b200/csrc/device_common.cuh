@@ -69,64 +69,80 @@ __device__ __forceinline__ float4 depth_entry(const View& V, int i, int j) {
     return __ldg(V.depth_lut + __ldg(V.pd + (size_t)i * V.w + j));
 }
 
-// L: depth_entry(V, i, j), loaded by the caller (the warp kernel issues a
-// thread's loads ahead of its arithmetic).  kErpOut: the output may be
-// equirectangular (compiled out of kernels whose outputs all are perspective).
-template <bool kErpOut, class View>
-__device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T, int i, int j, float4 L) {
+// What the views and the target of a launch can be; what they cannot is
+// compiled out of its mesh kernel.
+enum InputKind { kPerspectiveIn = 0, kErpIn = 1, kAnyIn = 2 };
+
+// What the unprojection of an input column needs, the same for all its rows.
+struct InputColumn {
+    float a, b;  // perspective: pixel centre - p0; equirectangular: cos, sin of phi
+};
+template <int kIn, class View>
+__device__ __forceinline__ InputColumn input_column(const View& V, int j) {
+    if (kIn == kErpIn || (kIn == kAnyIn && V.proj == 1)) return {V.erp_col[2 * j], V.erp_col[2 * j + 1]};
+    return {__fsub_rn(__fadd_rn((float)j, 0.5f), V.p0), 0.f};
+}
+
+// L: depth_entry(V, i, j), loaded by the caller (the mesh kernel issues a
+// thread's loads ahead of its arithmetic); col: input_column(V, j).
+template <int kIn, bool kErpOut, bool kScaled, class View>
+__device__ __forceinline__ float4 warp_vertex(const View& V, const DevTarget& T, int i, InputColumn col, float4 L) {
     const float d = L.x;
-    float x0, x1, x2;
-    if (V.proj == 1) {
+    float x0 = d, x1, x2;
+    // Invalid depths and points behind the camera become NaN at the end, by
+    // selection: a branch around the arithmetic would cost more than it saves.
+    bool ok = true;
+    if (kIn == kErpIn || (kIn == kAnyIn && V.proj == 1)) {
         const float ct = V.erp_row[2 * i], st = V.erp_row[2 * i + 1];
-        const float cp = V.erp_col[2 * j], sp = V.erp_col[2 * j + 1];
-        x0 = __fmul_rn(d, __fmul_rn(ct, cp));
-        x1 = __fmul_rn(d, __fmul_rn(ct, sp));
+        x0 = __fmul_rn(d, __fmul_rn(ct, col.a));
+        x1 = __fmul_rn(d, __fmul_rn(ct, col.b));
         x2 = __fmul_rn(d, st);
     } else {
-        const float pu = __fadd_rn((float)j, 0.5f), pv = __fadd_rn((float)i, 0.5f);
-        if (d > 0.f) {
-            x0 = d;
-            // L.y = -(d / f0), L.z = -(d / f1), divided once per sample
-            // value when the table was built.
-            x1 = __fmul_rn(L.y, __fsub_rn(pu, V.p0));
-            x2 = __fmul_rn(L.z, __fsub_rn(pv, V.p1));
-        } else {
-            x0 = x1 = x2 = qnan();
-        }
+        // L.y = -(d / f0), L.z = -(d / f1), divided once per sample
+        // value when the table was built.
+        x1 = __fmul_rn(L.y, col.a);
+        x2 = __fmul_rn(L.z, __fsub_rn(__fadd_rn((float)i, 0.5f), V.p1));
+        ok = d > 0.f;
     }
     float y[3];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        float s = __fadd_rn(0.f, __fmul_rn(V.R[r * 3 + 0], x0));
+        // The sum starts from 0, which turns -0 into +0: that shows only in
+        // the arctangent of an equirectangular output.
+        float s = __fmul_rn(V.R[r * 3 + 0], x0);
+        if (kErpOut) s = __fadd_rn(0.f, s);
         s = __fadd_rn(s, __fmul_rn(V.R[r * 3 + 1], x1));
         s = __fadd_rn(s, __fmul_rn(V.R[r * 3 + 2], x2));
         y[r] = __fadd_rn(s, V.t[r]);
     }
+    const float nan = qnan();
     float u, v, z;
     if (kErpOut && T.proj == 1) {
         float phi, theta;
+        if (!ok) y[0] = y[1] = y[2] = nan;
         erp_direction(y[0], y[1], y[2], z, phi, theta);
         u = __fadd_rn(T.u0, __fmul_rn(T.du_dphi, phi));
         v = __fadd_rn(T.v0, __fmul_rn(T.dv_dtheta, theta));
     } else {
-        if (y[0] > 0.f) {
-            u = __fadd_rn(__fdiv_rn(__fmul_rn(-T.f0, y[1]), y[0]), T.p0);
-            v = __fadd_rn(__fdiv_rn(__fmul_rn(-T.f1, y[2]), y[0]), T.p1);
-            z = y[0];
-        } else {
-            u = v = z = qnan();
-        }
+        ok = ok && y[0] > 0.f;
+        u = __fadd_rn(__fdiv_rn(__fmul_rn(-T.f0, y[1]), y[0]), T.p0);
+        v = __fadd_rn(__fdiv_rn(__fmul_rn(-T.f1, y[2]), y[0]), T.p1);
+        z = y[0];
     }
-    if (T.rescale) {
+    if (kScaled && T.rescale) {
         // cv::transform with Matx22f(sx, 0, 0, sy) (SynthesizedView.cpp:330-331)
         const float su = __fadd_rn(__fmul_rn(T.uv_sx, u), __fmul_rn(0.f, v));
         const float sv = __fadd_rn(__fmul_rn(0.f, u), __fmul_rn(T.uv_sy, v));
         u = su;
         v = sv;
     }
+    if (!(kErpOut && T.proj == 1)) {
+        u = ok ? u : nan;
+        v = ok ? v : nan;
+        z = ok ? z : nan;
+    }
     return make_float4(u, v, z, 0.f);
 }
-
 
 // Triangle quality of transform.cpp:62-75 (valid_tri): the longest edge by
 // cv::norm (double sum of squared float differences, double sqrt), then

@@ -345,6 +345,7 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
     BatchShape sh;
     sh.slots = n;
     sh.variant = variant;
+    bool persp = false, erp = false;
     for (int k = 0; k < n; ++k) {
         const SlotRequest& r = reqs[k];
         if (r.aux) sh.aux = 1;
@@ -356,6 +357,7 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
         for (const auto& c : r.scene->cams) {
             sh.max_w = std::max(sh.max_w, c.width);
             sh.max_h = std::max(sh.max_h, c.height);
+            (c.projection == RVSB_PROJ_EQUIRECTANGULAR ? erp : persp) = true;
         }
         const RasterDims rd = raster_dims(r.virt, r.params);
         sh.max_wo = std::max(sh.max_wo, rd.w);
@@ -363,6 +365,7 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
         sh.max_out_w = std::max(sh.max_out_w, r.virt.width);
         sh.max_out_h = std::max(sh.max_out_h, r.virt.height);
     }
+    sh.inputs = erp ? (persp ? 2 : 1) : 0;
     // The four words per pixel that the inpainting scans use later hold the
     // z-buffers of up to four views, or, for more views, of three at a time
     // and half of the running blend (its other half takes the codes').
@@ -392,7 +395,7 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
     const TablePtr tabs{tables_.as<SlotTable>()};
     if (use_graphs_ && !profiling_) {
         const std::vector<int> key = {sh.slots, sh.variant, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
-                                      sh.max_ho, sh.aux, sh.ms, sh.extras, sh.erp_out, sh.rescale, sh.max_out_w, sh.max_out_h};
+                                      sh.max_ho, sh.aux, sh.ms, sh.extras, sh.erp_out, sh.inputs, sh.rescale, sh.max_out_w, sh.max_out_h};
         auto it = graphs_.find(key);
         if (it == graphs_.end()) {
             cudaGraph_t g = nullptr;

@@ -289,7 +289,7 @@ struct LargeQueue {
 // Grid (ceil(strips / MESH_WARPS), ceil(max quad rows / rows), slots * gv):
 // views g0 .. g0 + gv - 1 of every slot.  ERP outputs wrapping horizontally
 // have one more strip, whose lanes take the seam triangles of one row each.
-template <int SMALL, bool kErpOut, class Tabs>
+template <int SMALL, int kIn, bool kErpOut, bool kScaled, class Tabs>
 __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_constant__ Tabs tabs, int g0, int gv,
                                                                    int rows) {
     __shared__ uint4 s_queue[MESH_WARPS][QUEUE];
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
     const int i1 = min(i0 + rows, G.h - 1);  // last vertex row of the warp's quads
     const int j = strip * STRIP + lane;
     bool keep_all = false;
-    if (T.cull && G.erp_cone) {
+    if (kIn != kPerspectiveIn && T.cull && G.erp_cone) {
         // Quad rows i0 .. i1 - 1 lie in one row of vertex tiles (rows divides
         // WARP_TILE) and the strip's quads in at most two tiles of it; every
         // quad's corners lie in its tile grown by one pixel.
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
     o.ymax = kBiasBits + T.ho - 1;
     o.z = G.z;
     o.origin = (uint32_t)kBiasBits * (uint32_t)T.wo + (uint32_t)kBiasBits;
-    o.precision = T.precision;
+    o.precision = kScaled ? T.precision : 1.f;
     float4* vert = G.vert;
     const int shift = G.tri_shift;
     LargeQueue queue{s_queue[warp], 0};
@@ -334,10 +334,12 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
         const bool in_col = j < V.w;
         const bool store = in_col && (lane < STRIP || j == V.w - 1 || keep_all);
         const int jc = min(j, V.w - 1);
+        const bool last = i1 == V.h - 1 || keep_all;  // row i1 is stored here
+        const InputColumn col = input_column<kIn>(V, jc);
         float4 L = depth_entry(V, i0, jc);
         uint16_t raw = __ldg(V.pd + (size_t)min(i0 + 2, i1) * V.w + jc);
         float4 Ln = depth_entry(V, i0 + 1, jc);
-        float4 a = warp_vertex<kErpOut>(V, T, i0, jc, L);
+        float4 a = warp_vertex<kIn, kErpOut, kScaled>(V, T, i0, col, L);
         if (store) vert[(size_t)i0 * V.w + j] = a;
         // Emission test (transform.cpp:161-167) per vertex, as masks of the row.
         unsigned ok_a = __ballot_sync(0xffffffffu, a.z > 0.f && a.x > 0.f);
@@ -348,8 +350,8 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
             L = Ln;
             Ln = __ldg(V.depth_lut + raw);
             raw = __ldg(V.pd + (size_t)min(i + 3, i1) * V.w + jc);
-            const float4 c = warp_vertex<kErpOut>(V, T, i + 1, jc, L);
-            if (store && (i + 1 < i1 || i1 == V.h - 1 || keep_all)) vert[(size_t)(i + 1) * V.w + j] = c;
+            const float4 c = warp_vertex<kIn, kErpOut, kScaled>(V, T, i + 1, col, L);
+            if (store && (i + 1 < i1 || last)) vert[(size_t)(i + 1) * V.w + j] = c;
             const unsigned ok_c = __ballot_sync(0xffffffffu, c.z > 0.f && c.x > 0.f);
             const float dx = __shfl_down_sync(0xffffffffu, c.x, 1), dy = __shfl_down_sync(0xffffffffu, c.y, 1),
                         dz = __shfl_down_sync(0xffffffffu, c.z, 1);
@@ -399,7 +401,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
 #pragma unroll 1
         for (int k = 0; k < 5; ++k) {
             const int r = i + (k == 2 || k == 4), q = k == 1 ? 1 : k >= 3 ? V.w - 1 : 0;
-            v[k] = warp_vertex<kErpOut>(V, T, r, q, depth_entry(V, r, q));
+            v[k] = warp_vertex<kIn, kErpOut, kScaled>(V, T, r, input_column<kIn>(V, q), depth_entry(V, r, q));
         }
         const float4 v00 = v[0], v01 = v[1], v10 = v[2], w0 = v[3], w1 = v[4];
         const bool active = i0 + lane < i1 && v01.z > 0.f && v10.z > 0.f && v01.x > 0.f && v10.x > 0.f;
@@ -748,7 +750,7 @@ static int rows_per_warp(const BatchShape& sh, int gv) {
     return warps < 2 * wave ? 4 : warps < 40 * wave ? 8 : 32;
 }
 
-template <bool kErpOut, class Tabs>
+template <int kIn, bool kErpOut, bool kScaled, class Tabs>
 static void launch_mesh_kernel(const Tabs& tabs, const BatchShape& sh, int g0, int gv, cudaStream_t s) {
     RasterVariant rv = kRasterVariants[sh.variant];
     if (rv.rows == 0) rv.rows = rows_per_warp(sh, gv);
@@ -756,9 +758,33 @@ static void launch_mesh_kernel(const Tabs& tabs, const BatchShape& sh, int g0, i
     const dim3 grid((strips + MESH_WARPS - 1) / MESH_WARPS, (sh.max_h - 1 + rv.rows - 1) / rv.rows, sh.slots * gv);
     auto go = [&](auto kernel) { launch_dependent(kernel, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); };
     switch (rv.small) {
-        case 4: go(mesh_kernel<4, kErpOut, Tabs>); break;
-        case 8: go(mesh_kernel<8, kErpOut, Tabs>); break;
-        default: go(mesh_kernel<16, kErpOut, Tabs>); break;
+        case 4: go(mesh_kernel<4, kIn, kErpOut, kScaled, Tabs>); break;
+        case 8: go(mesh_kernel<8, kIn, kErpOut, kScaled, Tabs>); break;
+        default: go(mesh_kernel<16, kIn, kErpOut, kScaled, Tabs>); break;
+    }
+}
+
+// The kernel instantiated for what the launch holds (without the projections
+// and the scaling that do not occur, and with a column's factors held across its
+// rows, it needs fewer registers and constants: 4 x 1920x1080 193 -> 173 us the
+// stage, into 960x540 152 -> 134, 8 poses 160 -> 149 us a view); the rarer
+// mixtures share general ones.
+template <class Tabs>
+static void launch_mesh_kernels(const Tabs& tabs, const BatchShape& sh, int g0, int gv, cudaStream_t s) {
+    if (sh.erp_out) {
+        if (sh.inputs == kErpIn && !sh.rescale)
+            launch_mesh_kernel<kErpIn, true, false>(tabs, sh, g0, gv, s);
+        else
+            launch_mesh_kernel<kAnyIn, true, true>(tabs, sh, g0, gv, s);
+    } else if (sh.inputs == kPerspectiveIn) {
+        if (sh.rescale)
+            launch_mesh_kernel<kPerspectiveIn, false, true>(tabs, sh, g0, gv, s);
+        else
+            launch_mesh_kernel<kPerspectiveIn, false, false>(tabs, sh, g0, gv, s);
+    } else if (sh.inputs == kErpIn && !sh.rescale) {
+        launch_mesh_kernel<kErpIn, false, false>(tabs, sh, g0, gv, s);
+    } else {
+        launch_mesh_kernel<kAnyIn, false, true>(tabs, sh, g0, gv, s);
     }
 }
 
@@ -769,10 +795,7 @@ int launch_mesh(const Tabs& tabs, const BatchShape& sh, int g0, cudaStream_t s, 
     if (ev) cudaEventRecord(ev[0], s);
     launch_dependent(clear_kernel<Tabs>, dim3((unsigned)std::min<size_t>(2048, (words / 2 + 255) / 256 + 1), sh.slots),
                      dim3(256), 0, s, tabs, g0, gv);
-    if (sh.erp_out)
-        launch_mesh_kernel<true>(tabs, sh, g0, gv, s);
-    else
-        launch_mesh_kernel<false>(tabs, sh, g0, gv, s);
+    launch_mesh_kernels(tabs, sh, g0, gv, s);
     if (ev) {
         cudaEventRecord(ev[1], s);
         cudaEventRecord(ev[2], s);

@@ -64,3 +64,25 @@ def test_large_triangle_list_overflow(ctx, erp_in):
         target = _resized(wl.targets[0], 384, 288)
     yuv = _each_variant(ctx, wl, target, [0, 7])
     assert_parity(yuv, O.synthesize(wl.inputs, wl.planes, target, 5.0))
+
+
+@pytest.mark.parametrize("precision", [1.0, 1.5])
+@pytest.mark.parametrize("erp_out", [False, True], ids=["persp_out", "erp_out"])
+@pytest.mark.parametrize("inputs", ["erp", "mixed"])
+def test_projection_mixtures(ctx, inputs, erp_out, precision):
+    """The instantiations of the mesh kernel by what a launch holds:
+    equirectangular inputs alone and beside a perspective one, both kinds of
+    output, with and without Precision."""
+    wl = scenes.random_pose_small(n_views=2, w=128, h=64, seed=320, erp_in=True, erp_out=erp_out)
+    if inputs == "mixed":
+        flat = scenes.random_pose_small(n_views=1, w=96, h=54, seed=321)
+        wl.inputs.append(flat.inputs[0])
+        wl._planes = list(wl.planes[:2]) + [flat.planes[0]]
+    p = rvsb.params(5.0, precision=precision)
+    yuv, _ = gpu_synthesize(ctx, wl.inputs, wl.planes, wl.targets[0], 5.0, params=p)
+    O.set_precision(precision)
+    try:
+        cpu = O.synthesize(wl.inputs, wl.planes, wl.targets[0], 5.0)
+    finally:
+        O.set_precision(1.0)
+    assert_parity(yuv, cpu)
