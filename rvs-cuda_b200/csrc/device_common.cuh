@@ -322,32 +322,33 @@ __device__ __forceinline__ float3 input_color(const DevView& V, int x, int y) {
 // exponents are evaluated as a double product and rounded once, which is
 // the correctly rounded result except within about 2^-28 of a rounding
 // boundary.
+__device__ __forceinline__ float int_pow(float x, int e_int) {
+    // e_int - 1 multiplications: the exponent is the same for all pixels,
+    // so the jump is uniform.
+    const double b = (double)x;
+    double r = b;
+    switch (e_int) {
+        case 16: r = __dmul_rn(r, b); [[fallthrough]];
+        case 15: r = __dmul_rn(r, b); [[fallthrough]];
+        case 14: r = __dmul_rn(r, b); [[fallthrough]];
+        case 13: r = __dmul_rn(r, b); [[fallthrough]];
+        case 12: r = __dmul_rn(r, b); [[fallthrough]];
+        case 11: r = __dmul_rn(r, b); [[fallthrough]];
+        case 10: r = __dmul_rn(r, b); [[fallthrough]];
+        case 9: r = __dmul_rn(r, b); [[fallthrough]];
+        case 8: r = __dmul_rn(r, b); [[fallthrough]];
+        case 7: r = __dmul_rn(r, b); [[fallthrough]];
+        case 6: r = __dmul_rn(r, b); [[fallthrough]];
+        case 5: r = __dmul_rn(r, b); [[fallthrough]];
+        case 4: r = __dmul_rn(r, b); [[fallthrough]];
+        case 3: r = __dmul_rn(r, b); [[fallthrough]];
+        default: r = __dmul_rn(r, b);
+    }
+    return __double2float_rn(r);
+}
 __device__ __forceinline__ float blend_pow(float x, float e, int e_int) {
     if (e == 1.f) return x;
-    if (e_int > 0) {
-        // e_int - 1 multiplications: the exponent is the same for all pixels,
-        // so the jump is uniform.
-        const double b = (double)x;
-        double r = b;
-        switch (e_int) {
-            case 16: r = __dmul_rn(r, b); [[fallthrough]];
-            case 15: r = __dmul_rn(r, b); [[fallthrough]];
-            case 14: r = __dmul_rn(r, b); [[fallthrough]];
-            case 13: r = __dmul_rn(r, b); [[fallthrough]];
-            case 12: r = __dmul_rn(r, b); [[fallthrough]];
-            case 11: r = __dmul_rn(r, b); [[fallthrough]];
-            case 10: r = __dmul_rn(r, b); [[fallthrough]];
-            case 9: r = __dmul_rn(r, b); [[fallthrough]];
-            case 8: r = __dmul_rn(r, b); [[fallthrough]];
-            case 7: r = __dmul_rn(r, b); [[fallthrough]];
-            case 6: r = __dmul_rn(r, b); [[fallthrough]];
-            case 5: r = __dmul_rn(r, b); [[fallthrough]];
-            case 4: r = __dmul_rn(r, b); [[fallthrough]];
-            case 3: r = __dmul_rn(r, b); [[fallthrough]];
-            default: r = __dmul_rn(r, b);
-        }
-        return __double2float_rn(r);
-    }
+    if (e_int > 0) return int_pow(x, e_int);
     return powf(x, e);
 }
 

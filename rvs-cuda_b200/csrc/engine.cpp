@@ -351,6 +351,8 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
         if (r.aux) sh.aux = 1;
         if (r.params.blending_method == RVSB_BLEND_MULTISPECTRAL) sh.ms = 1;
         if (r.params.precision != 1.f) sh.rescale = 1;
+        const float e = r.params.blending_factor;
+        if (!(e == std::floor(e) && e >= 2.f && e <= 16.f)) sh.int_pow = 0;
         if (r.virt.projection == RVSB_PROJ_EQUIRECTANGULAR) sh.erp_out = 1;
         if (r.aux || r.dbg.any() || r.params.blending_method == RVSB_BLEND_MULTISPECTRAL) sh.extras = 1;
         sh.max_views = std::max(sh.max_views, (int)r.scene->cams.size());
@@ -395,7 +397,7 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
     const TablePtr tabs{tables_.as<SlotTable>()};
     if (use_graphs_ && !profiling_) {
         const std::vector<int> key = {sh.slots, sh.variant, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
-                                      sh.max_ho, sh.aux, sh.ms, sh.extras, sh.erp_out, sh.inputs, sh.rescale, sh.max_out_w, sh.max_out_h};
+                                      sh.max_ho, sh.aux, sh.ms, sh.extras, sh.erp_out, sh.int_pow, sh.inputs, sh.rescale, sh.max_out_w, sh.max_out_h};
         auto it = graphs_.find(key);
         if (it == graphs_.end()) {
             cudaGraph_t g = nullptr;

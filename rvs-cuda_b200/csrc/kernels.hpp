@@ -16,6 +16,7 @@ struct BatchShape {
     int aux = 0;             // some slot wants auxiliary outputs
     int ms = 0;              // some slot blends multispectrally
     int erp_out = 0;         // some output is equirectangular
+    int int_pow = 1;         // every blending exponent is an integer from 2 to 16
     int inputs = 0;          // input views: 0 all perspective, 1 all equirectangular, 2 both
     int extras = 0;          // some slot wants per-view, auxiliary or debug outputs of the resolve
     int max_views = 0;       // largest n_views

@@ -80,7 +80,8 @@ __device__ __forceinline__ float tri_quality_fast(float4 A, float4 B, float4 C, 
 
 // Re-evaluates the winning triangle at pixel (x, y) exactly as the CPU's
 // colorize_triangle does for the fragment it keeps (transform.cpp:109-135).
-template <class View>
+// kWrap: seam triangles may occur; kScaled: Precision may differ from 1.
+template <bool kWrap, bool kScaled, class View>
 __device__ __forceinline__ Fragment resolve_fragment(const View& V, unsigned long long key, int x, int y,
                                                      float precision = 1.f) {
     Fragment f;
@@ -97,7 +98,7 @@ __device__ __forceinline__ Fragment resolve_fragment(const View& V, unsigned lon
     uint32_t a = q, b = q + 1u, c = q + w;
     if (t == 1u) {
         a = q + w + 1u; b = q + w; c = q + 1u;
-    } else if (t > 1u) {
+    } else if (kWrap && t > 1u) {
         int ax, ay, bx, by, cx, cy;
         tri_vertices(V.w, (int)i, (int)j, (int)t, ax, ay, bx, by, cx, cy);
         a = (uint32_t)ay * w + (uint32_t)ax;
@@ -114,7 +115,7 @@ __device__ __forceinline__ Fragment resolve_fragment(const View& V, unsigned lon
     f.col.y = interp(ca.y, cb.y, cc.y, l1, l2, l3);
     f.col.z = interp(ca.z, cb.z, cc.z, l1, l2, l3);
     f.depth = interp(A.z, B.z, C.z, l1, l2, l3);
-    f.validity = tri_quality_fast(A, B, C, precision);
+    f.validity = tri_quality_fast(A, B, C, kScaled ? precision : 1.f);
     return f;
 }
 
@@ -131,6 +132,8 @@ struct BlendAcc {
 // weight sum itself: the reference re-powers its stored sum^(1/exp) by exp,
 // which returns the sum up to a few ulp, and quality > 0 exactly when the
 // sum is > 0.
+// kIntPow: the exponent is an integer from 2 to 16 (and not by_max).
+template <bool kIntPow = false>
 __device__ __forceinline__ void blend_view(BlendAcc& a, int v, float3 col, float qv, float blend_exp, int exp_int,
                                            bool by_max) {
     if (v == 0) {
@@ -140,7 +143,7 @@ __device__ __forceinline__ void blend_view(BlendAcc& a, int v, float3 col, float
         a.q = qv;
         return;
     }
-    if (by_max) {
+    if (!kIntPow && by_max) {
         // blend_img_by_max (blending.cpp:293-308): the empty colour and
         // quality 0, replaced by the accumulator where its quality is
         // positive, then by the view where its quality is larger still.
@@ -157,14 +160,14 @@ __device__ __forceinline__ void blend_view(BlendAcc& a, int v, float3 col, float
     }
     float sum = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
     if (a.q > 0.f) {
-        const float w = v == 1 ? blend_pow(a.q, blend_exp, exp_int) : a.q;
+        const float w = v != 1 ? a.q : kIntPow ? int_pow(a.q, exp_int) : blend_pow(a.q, blend_exp, exp_int);
         sum = __fadd_rn(sum, w);
         c0 = __fadd_rn(c0, __fmul_rn(w, a.c0));
         c1 = __fadd_rn(c1, __fmul_rn(w, a.c1));
         c2 = __fadd_rn(c2, __fmul_rn(w, a.c2));
     }
     if (qv > 0.f) {
-        const float w = blend_pow(qv, blend_exp, exp_int);
+        const float w = kIntPow ? int_pow(qv, exp_int) : blend_pow(qv, blend_exp, exp_int);
         sum = __fadd_rn(sum, w);
         c0 = __fadd_rn(c0, __fmul_rn(w, col.x));
         c1 = __fadd_rn(c1, __fmul_rn(w, col.y));
@@ -182,8 +185,9 @@ __device__ __forceinline__ void blend_view(BlendAcc& a, int v, float3 col, float
     }
 }
 
+template <bool kIntPow>
 __device__ __forceinline__ void blend_view(BlendAcc& a, int v, const Fragment& f, float qv, const DevTarget& T) {
-    blend_view(a, v, f.col, qv, T.blend_exp, T.blend_exp_int, T.blend_max != 0);
+    blend_view<kIntPow>(a, v, f.col, qv, T.blend_exp, T.blend_exp_int, T.blend_max != 0);
 }
 
 }  // namespace dev
