@@ -786,19 +786,21 @@ def main():
     n_out = wo * ho
     stage_avg = {k: v / args.steps for k, v in stage_acc.items()}
     stage_avg["upload_decode"] = statistics.mean(step_ms) - stage_avg["total"]
-    # Algorithmic bytes per launch: warp 14 B per input pixel (depth read +
-    # warped u, v, z write); the raster kernel reads the warped mesh (12 B
-    # per input pixel) and, with the blend fused into it, (10N + 4) B per
-    # output pixel (per view colour 3 x u16 + weight fp32, output YUV420 +
-    # mask); the inpainting passes are charged the output write (4 B per
-    # output pixel).
+    # Algorithmic bytes per launch: the mesh kernel (stage warp) reads the depth
+    # samples and stores the warped u, v, z (14 B per input pixel) and takes
+    # the least key of every view and output pixel (8 B); the resolve (stage
+    # raster) reads those keys and the warped mesh (12 B per input pixel) and
+    # blends (10N + 4) B per output pixel (per view colour 3 x u16 + weight
+    # fp32, output YUV420 + mask); the inpainting passes are charged the
+    # output write (4 B per output pixel).
     blend_bytes = (10 * n_views + 4) * n_out
+    key_bytes = 8 * n_views * n_out
     algorithmic = {
-        "warp": 14 * n_in,
-        "raster": 12 * n_in + blend_bytes,
+        "warp": 14 * n_in + key_bytes,
+        "raster": 12 * n_in + key_bytes + blend_bytes,
         "inpaint": 4 * n_out,
     }
-    kernel_names = {"warp": "warp_kernel", "raster": "raster_kernel", "inpaint": "inpaint_*_kernel"}
+    kernel_names = {"warp": "mesh_kernel", "raster": "resolve_kernel", "inpaint": "inpaint_*_kernel"}
     dominant = max(("warp", "bin", "raster", "inpaint"), key=lambda k: stage_avg[k])
     peak, peak_kind = measured_peaks()
     rk = dominant if dominant in algorithmic else "raster"
@@ -819,7 +821,7 @@ def main():
                       "frac": algorithmic[k] / (stage_avg[k] / 1000.0) / 1e9 / peak}
                   for k in algorithmic}
     triangles = 2 * sum((c.width - 1) * (c.height - 1) for c in wl.inputs)
-    stage_roof["raster"]["triangles_per_s"] = triangles / (stage_avg["raster"] / 1000.0)
+    stage_roof["warp"]["triangles_per_s"] = triangles / (stage_avg["warp"] / 1000.0)
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:

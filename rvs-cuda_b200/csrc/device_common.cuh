@@ -60,7 +60,7 @@ __device__ __forceinline__ float decode_depth_raw(float near_, float far_, float
 // PerspectiveUnprojector.cpp:59-86 / EquirectangularUnprojector.cpp:55-98,
 // SynthesizedView.cpp:68-79 and PerspectiveProjector.cpp:59-87 /
 // EquirectangularProjector.cpp:60-99.
-// View: DevView, or a copy of the fields used here (the warp kernel keeps
+// View: DevView, or a copy of the fields used here (the mesh kernel keeps
 // them in registers).
 // The depth-table entry of input pixel (i, j): the decoded depth and the
 // perspective factors of its raw sample.

@@ -32,9 +32,9 @@
 // minimum of the groups' minima before it.  The stage is a chain of five
 // short kernels, bound by their latency at one image: against scans over
 // every pixel of the holes' bounding box (seven kernels, about 100 bytes a
-// pixel) a 1920x1080 view with holes along its borders takes 38 us instead of
-// 79, a 960x540 one 27 instead of 38, an equirectangular 4096x2048 one 60
-// instead of 214, and a batch of 8 1920x1080 views 24 us a view instead of 60.
+// pixel) a 1920x1080 view with holes along its borders takes 37 us instead of
+// 79, a 960x540 one 26 instead of 38, an equirectangular 4096x2048 one 52
+// instead of 214, and a batch of 8 1920x1080 views 21 us a view instead of 60.
 #include <algorithm>
 
 #include "device_common.cuh"

@@ -146,8 +146,8 @@ struct Tri {
 // overlaps, and one loop runs over the candidates of both (measured with the
 // perspective-only instantiation against one triangle after the other: 164 ->
 // 148 M warp instructions on 4 x 1920x1080 -> 1920x1080, the stage 233 -> 196
-// us, 200 -> 160 us a view in a batch of 8).  The kernel is bound by
-// instruction issue (82% of cycles); the atomics take no time of their own
+// us, 200 -> 160 us a view in a batch of 8; now 138 M, 164 and 149).  The kernel
+// is bound by instruction issue (87% of cycles); the atomics take no time of their own
 // (without them 191 us).
 //
 // Candidate range: a covered pixel's centre lies within the bounding box

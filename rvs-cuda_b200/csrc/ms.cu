@@ -1,5 +1,5 @@
 // Multispectral blending (BlendedViewMultiSpec, rvs/src/BlendedView.cpp:63-88),
-// after the raster has stored every view's resolved colour and quality:
+// after the resolve has stored every view's resolved colour and quality:
 // split_frequencies (blending.cpp:371-395; YUV: only luma is blurred) with
 // calcBlurring (blending.cpp:62-105: box mean over the masked pixels of a
 // (2r+1)^2 window clipped to the image, r = max(W, H) / 20, the window sum

@@ -8,11 +8,12 @@
 // colours through L1.
 //
 // Bound by instruction issue and the latency of the gathers (three vertices,
-// three colours per pixel and view) together: 4 views of 1920x1080 take 111
+// three colours per pixel and view) together: 4 views of 1920x1080 take 105
 // us (8.3 M pixel-views; their keys, vertices and colours, each read once,
-// are 265 MB, 41 us), 105 us a view in a batch of 8.  Five CTAs per SM at 48
-// registers beat four at 64 (batch 107 against 117 us), two views' gathers in
-// flight per thread (116) and six CTAs at 40 registers (112).
+// are 265 MB, 41 us), 97 us a view in a batch of 8.  Five CTAs per SM at 48
+// registers beat four at 64 (in one kernel for all options: batch 107 against
+// 117 us), two views' gathers in flight per thread (116) and six CTAs at 40
+// registers (112).
 #include <algorithm>
 
 #include "device_common.cuh"

@@ -1,4 +1,4 @@
-// Resolve and blend of one output pixel, used by the raster kernel once a
+// Resolve and blend of one output pixel, used by the resolve kernel once a
 // view's z-buffer is final: re-evaluate the winning fragment exactly, fold it
 // into the running blend in blend order (BlendedViewSimple::blendBasicMode +
 // blend_img, BlendedView.cpp:180-212, blending.cpp:310-369).
