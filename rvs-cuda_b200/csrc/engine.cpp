@@ -341,6 +341,56 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     }
 }
 
+namespace {
+
+// Pixels per radian at the centre of a camera: the focal length of a
+// perspective camera, the width over the horizontal range of an
+// equirectangular one.
+float pixels_per_radian(const rvsb_camera& c) {
+    if (c.projection == RVSB_PROJ_EQUIRECTANGULAR) {
+        const float range = (c.hor_range[1] - c.hor_range[0]) * (3.14159265f / 180.f);
+        return range > 0.f ? (float)c.width / range : 0.f;
+    }
+    return c.focal[0];
+}
+
+// Largest magnification of a batch: output pixels per radian at the raster size
+// over the densest input's.  An equirectangular output stretches its rows by
+// 1 / cos(latitude), sqrt(2) at the median row, which its m includes.
+float magnification(const SlotRequest* reqs, int n, bool& erp_out) {
+    float m = 0.f;
+    erp_out = false;
+    for (int k = 0; k < n; ++k) {
+        const SlotRequest& r = reqs[k];
+        float in = 0.f;
+        for (const rvsb_camera& c : r.scene->cams) in = std::max(in, pixels_per_radian(c));
+        const RasterDims rd = raster_dims(r.virt, r.params);
+        float out = pixels_per_radian(r.virt) * (float)rd.w / (float)r.virt.width;
+        if (r.virt.projection == RVSB_PROJ_EQUIRECTANGULAR) {
+            out *= 1.41421356f;
+            erp_out = true;
+        }
+        if (in > 0.f) m = std::max(m, out / in);
+    }
+    return m;
+}
+
+// Candidate pixels up to which a magnified view's triangles stay with their
+// lanes.  An input pixel spacing seen m times magnified gives candidate boxes
+// of about m + 1 pixels a side, somewhat more where the surface is slanted.  A
+// threshold below that lists nearly every triangle, which overflows the list:
+// 3 x ERP 1102x550 into ERP 3890x1944 (m = 5) 1303 us with 16, 724 with 49; 2 x
+// 480x270 into 1920x1080 (m = 4) 211 with 16, 146 with 25, 149 with 36; 4 x
+// 240x136 (m = 8) 509 with 64, 244 with 100.  One far above it leaves stretched
+// triangles to single lanes: m = 2, 193 us with 9 and 16, 211 with 36, 270 with
+// 120.  Below 16 nothing is gained (m = 1.5, 224 us with 4 to 16).
+int magnified_threshold(float m) {
+    const int side = (int)std::min(20.f, std::max(4.f, std::ceil(m + 1.2f)));
+    return side * side;
+}
+
+}  // namespace
+
 BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) const {
     BatchShape sh;
     sh.slots = n;
@@ -368,6 +418,9 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
         sh.max_out_h = std::max(sh.max_out_h, r.virt.height);
     }
     sh.inputs = erp ? (persp ? 2 : 1) : 0;
+    bool erp_out;
+    sh.small = kRasterVariants[variant].small;
+    if (sh.small == 0) sh.small = magnified_threshold(magnification(reqs, n, erp_out));
     // The four words per pixel that the inpainting scans use later hold the
     // z-buffers of up to four views, or, for more views, of three at a time
     // and half of the running blend (its other half takes the codes').
@@ -396,7 +449,7 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
     cur_ ^= 1;
     const TablePtr tabs{tables_.as<SlotTable>()};
     if (use_graphs_ && !profiling_) {
-        const std::vector<int> key = {sh.slots, sh.variant, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
+        const std::vector<int> key = {sh.slots, sh.variant, sh.small, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
                                       sh.max_ho, sh.aux, sh.ms, sh.extras, sh.erp_out, sh.int_pow, sh.inputs, sh.rescale, sh.max_out_w, sh.max_out_h};
         auto it = graphs_.find(key);
         if (it == graphs_.end()) {
@@ -422,30 +475,16 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
 
 namespace {
 
-// Pixels per radian at the centre of a camera: the focal length of a
-// perspective camera, the width over the horizontal range of an
-// equirectangular one.
-float pixels_per_radian(const rvsb_camera& c) {
-    if (c.projection == RVSB_PROJ_EQUIRECTANGULAR) {
-        const float range = (c.hor_range[1] - c.hor_range[0]) * (3.14159265f / 180.f);
-        return range > 0.f ? (float)c.width / range : 0.f;
-    }
-    return c.focal[0];
-}
-
-// Raster variant of a run that is neither pinned nor tuned.  An input pixel
-// spacing seen m times magnified in the raster gives triangles whose
-// candidate boxes hold about (m + 1)^2 pixels: at m = 1 one or two, and then
-// the few above 4 go to the list of large triangles; past m of about 1.1 the
-// threshold is 16, so that the ordinary triangles stay with their lanes: 2 x
-// 960x540 into 1920x1080 (m = 2) 158 us against 249 with 4, 8 views of 4 ERP
-// 4096x2048 inputs (m = 1.47) 2.06 ms against 2.75.  At m <= 1 a threshold of
-// 16 costs up to 6% (4 x 1920x1080 into 960x540 245 us against 232).  An
-// equirectangular output stretches its rows by 1 / cos(latitude), sqrt(2) at
-// the median row, which its m includes (4 x ERP 4096x2048 into the same: 1.67
-// ms against 1.81).  The largest m of the batch decides.  The unmagnified
-// classes (one view, one minified to m <= 0.6, a batch of 8 or more) share
-// their parameters; the rows per warp follow the launch's size (mesh.cu).
+// Raster variant of a run that is neither pinned nor tuned.  At a magnification
+// of m = 1 a triangle has one or two candidates, and the few above 4 go to the
+// list of large triangles; past m of about 1.1 the threshold follows m
+// (magnified_threshold), so that the ordinary triangles stay with their lanes:
+// 2 x 960x540 into 1920x1080 (m = 2) 158 us against 249 with 4, 8 views of 4
+// ERP 4096x2048 inputs (m = 1.47) 2.06 ms against 2.75, 4 x ERP 4096x2048 into
+// the same 1.67 ms against 1.81.  At m <= 1 a threshold of 16 costs up to 6%
+// (4 x 1920x1080 into 960x540 245 us against 232).  The unmagnified classes
+// (one view, one minified to m <= 0.6, a batch of 8 or more) share their
+// parameters; the rows per warp follow the launch's size (mesh.cu).
 constexpr int kMagnifiedVariant = 7;
 constexpr int kDefaultVariant = 4;
 constexpr int kMinifiedVariant = 2;
@@ -453,20 +492,8 @@ constexpr int kBatchVariant = 1;
 constexpr int kBatchVariantMinSlots = 8;
 
 int default_variant(const SlotRequest* reqs, int n) {
-    float m = 0.f;
-    bool erp_out = false;
-    for (int k = 0; k < n; ++k) {
-        const SlotRequest& r = reqs[k];
-        float in = 0.f;
-        for (const rvsb_camera& c : r.scene->cams) in = std::max(in, pixels_per_radian(c));
-        const RasterDims rd = raster_dims(r.virt, r.params);
-        float out = pixels_per_radian(r.virt) * (float)rd.w / (float)r.virt.width;
-        if (r.virt.projection == RVSB_PROJ_EQUIRECTANGULAR) {
-            out *= 1.41421356f;
-            erp_out = true;
-        }
-        if (in > 0.f) m = std::max(m, out / in);
-    }
+    bool erp_out;
+    const float m = magnification(reqs, n, erp_out);
     if (m > 1.1f) return kMagnifiedVariant;
     if (!erp_out && m <= 0.6f) return kMinifiedVariant;
     return n >= kBatchVariantMinSlots ? kBatchVariant : kDefaultVariant;

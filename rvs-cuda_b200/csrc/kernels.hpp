@@ -13,6 +13,7 @@ namespace rvsb {
 struct BatchShape {
     int slots = 0;
     int variant = 0;         // raster variant (kRasterVariants)
+    int small = 0;           // candidate pixels above which a triangle goes to the list
     int aux = 0;             // some slot wants auxiliary outputs
     int ms = 0;              // some slot blends multispectrally
     int erp_out = 0;         // some output is equirectangular
@@ -76,26 +77,20 @@ int launch_batch(const Tabs& tabs, const BatchShape& shape, cudaStream_t stream,
 
 // Raster variants the autotuner chooses from: quad rows per warp of the mesh
 // kernel (0: by the launch's size) and the candidate pixels above which a
-// triangle goes to the list of large ones.  Every variant gives identical
+// triangle goes to the list of large ones (0: by the magnification).  Every variant gives identical
 // results.
 struct RasterVariant {
     int rows, small;
 };
 constexpr int NUM_RASTER_VARIANTS = 8;
 constexpr RasterVariant kRasterVariants[NUM_RASTER_VARIANTS] = {
-    {4, 4}, {0, 4}, {0, 4}, {8, 8}, {0, 4}, {16, 4}, {32, 16}, {0, 16},
+    {4, 4}, {0, 4}, {0, 4}, {8, 8}, {0, 4}, {16, 4}, {32, 16}, {0, 0},
 };
 constexpr bool rows_divide_tiles() {
     for (const RasterVariant& v : kRasterVariants)
         if (v.rows != 0 && WARP_TILE % v.rows != 0) return false;
     return true;
 }
-constexpr bool small_has_kernel() {
-    for (const RasterVariant& v : kRasterVariants)
-        if (v.small != 4 && v.small != 8 && v.small != 16) return false;
-    return true;
-}
-static_assert(small_has_kernel(), "a threshold without an instantiation of the mesh kernel");
 static_assert(rows_divide_tiles(), "a warp's quad rows must lie in one row of culling tiles");
 
 // Shared memory of the multispectral row sums for outputs up to max_wo wide.

@@ -19,7 +19,7 @@
 // mesh_kernel: one warp takes a strip of 32 vertex columns (31 quads) and
 // `rows` rows of quads, a lane one column: it warps the row below, gets the
 // right neighbour's vertices by shuffles, and rasterises the two triangles of
-// its quad.  Triangles of up to SMALL candidate pixels are tested by their
+// its quad.  Triangles of up to `small` candidate pixels are tested by their
 // lane; larger ones (stretched over depth discontinuities) go to the slot's
 // list and large_kernel rasterises them, one warp per entry, lanes over the
 // pixels of their row spans.
@@ -162,8 +162,8 @@ struct Tri {
 // one of 21u * M, so for M < 24/21 the constant 24u still holds; and since
 // the three coordinates add up to 1, M >= 24/21 puts the smallest below
 // -(M - 1) / 2 < -0.07, far outside.
-template <int SMALL, int N>
-__device__ __forceinline__ void raster_small(const MeshTarget& o, Tri (&t)[N], uint32_t tri) {
+template <int N>
+__device__ __forceinline__ void raster_small(const MeshTarget& o, Tri (&t)[N], uint32_t tri, int small) {
     const float u = 5.9604645e-8f, eps = 1e-6f;
     float den[N];
     int n[N], nmax = 0;
@@ -179,7 +179,7 @@ __device__ __forceinline__ void raster_small(const MeshTarget& o, Tri (&t)[N], u
         t[k].box.w = min(o.ymax, __float_as_int(__fadd_rn(__fadd_rn(t[k].mxy, delta), kBias)) - 1);
         const bool some = t[k].active && den[k] > 0.f && t[k].box.x <= t[k].box.z && t[k].box.y <= t[k].box.w;
         const int count = (t[k].box.z - t[k].box.x + 1) * (t[k].box.w - t[k].box.y + 1);
-        const bool own = !t[k].wide && count <= SMALL && den[k] >= 1e-30f;
+        const bool own = !t[k].wide && count <= small && den[k] >= 1e-30f;
         t[k].large = some && !own;
         n[k] = some && own ? count : 0;
         nmax = max(nmax, n[k]);
@@ -289,9 +289,9 @@ struct LargeQueue {
 // Grid (ceil(strips / MESH_WARPS), ceil(max quad rows / rows), slots * gv):
 // views g0 .. g0 + gv - 1 of every slot.  ERP outputs wrapping horizontally
 // have one more strip, whose lanes take the seam triangles of one row each.
-template <int SMALL, int kIn, bool kErpOut, bool kScaled, class Tabs>
+template <int kIn, bool kErpOut, bool kScaled, class Tabs>
 __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_constant__ Tabs tabs, int g0, int gv,
-                                                                   int rows) {
+                                                                   int rows, int small) {
     __shared__ uint4 s_queue[MESH_WARPS][QUEUE];
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z / gv);
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
                 t[1].mnx = fminf(nx, dx); t[1].mxx = fmaxf(xx, dx);
                 t[1].mny = fminf(ny, dy); t[1].mxy = fmaxf(xy, dy);
                 t[1].m2 = fmaxf(md, fmaxf(sq2(t[1].a0c0, t[1].c1a1), sq2(__fsub_rn(dx, c.x), __fsub_rn(dy, c.y))));
-                raster_small<SMALL>(o, t, tri);
+                raster_small(o, t, tri, small);
                 if (__any_sync(0xffffffffu, t[0].large || t[1].large)) {
                     queue.push(tab.b, lane, t[0].large, tri, view, t[0].wide, t[0].box);
                     queue.push(tab.b, lane, t[1].large, tri + 1u, view, t[1].wide, t[1].box);
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
             s[0].mny = fminf(fminf(A.y, B.y), C.y); s[0].mxy = fmaxf(fmaxf(A.y, B.y), C.y);
             s[0].m2 = fmaxf(sq2(s[0].c0b0, s[0].b1c1), fmaxf(sq2(s[0].a0c0, s[0].c1a1),
                                                              sq2(__fsub_rn(A.x, B.x), __fsub_rn(A.y, B.y))));
-            raster_small<SMALL>(o, s, tri + (uint32_t)t);
+            raster_small(o, s, tri + (uint32_t)t, small);
             queue.push(tab.b, lane, s[0].large, tri + (uint32_t)t, view, s[0].wide, s[0].box);
         }
     }
@@ -752,16 +752,11 @@ static int rows_per_warp(const BatchShape& sh, int gv) {
 
 template <int kIn, bool kErpOut, bool kScaled, class Tabs>
 static void launch_mesh_kernel(const Tabs& tabs, const BatchShape& sh, int g0, int gv, cudaStream_t s) {
-    RasterVariant rv = kRasterVariants[sh.variant];
-    if (rv.rows == 0) rv.rows = rows_per_warp(sh, gv);
+    const int fixed = kRasterVariants[sh.variant].rows, rows = fixed ? fixed : rows_per_warp(sh, gv);
     const int strips = (sh.max_w - 1 + STRIP - 1) / STRIP + (kErpOut ? 1 : 0);  // and the seam's
-    const dim3 grid((strips + MESH_WARPS - 1) / MESH_WARPS, (sh.max_h - 1 + rv.rows - 1) / rv.rows, sh.slots * gv);
-    auto go = [&](auto kernel) { launch_dependent(kernel, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rv.rows); };
-    switch (rv.small) {
-        case 4: go(mesh_kernel<4, kIn, kErpOut, kScaled, Tabs>); break;
-        case 8: go(mesh_kernel<8, kIn, kErpOut, kScaled, Tabs>); break;
-        default: go(mesh_kernel<16, kIn, kErpOut, kScaled, Tabs>); break;
-    }
+    const dim3 grid((strips + MESH_WARPS - 1) / MESH_WARPS, (sh.max_h - 1 + rows - 1) / rows, sh.slots * gv);
+    launch_dependent(mesh_kernel<kIn, kErpOut, kScaled, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rows,
+                     sh.small);
 }
 
 // The kernel instantiated for what the launch holds (without the projections

@@ -66,6 +66,23 @@ def test_large_triangle_list_overflow(ctx, erp_in):
     assert_parity(yuv, O.synthesize(wl.inputs, wl.planes, target, 5.0))
 
 
+# Thresholds of magnified views: 16, 36, 49 and 400 candidates (the largest).
+@pytest.mark.parametrize("mag", [1.5, 4, 5.5, 24])
+@pytest.mark.parametrize("erp", [False, True], ids=["persp", "erp"])
+def test_threshold_follows_magnification(ctx, erp, mag):
+    """Every triangle in its lane (variant 7) against nearly every one in the
+    list or, when that overflows, taken from the mesh (variant 0), and the
+    oracle."""
+    wl = scenes.random_pose_small(n_views=2, w=64, h=32, seed=330, erp_in=erp, erp_out=erp)
+    if erp:
+        target = copy.deepcopy(wl.targets[0])
+        target.width, target.height = int(64 * mag), int(32 * mag)
+    else:
+        target = _resized(wl.targets[0], int(64 * mag), int(32 * mag))
+    yuv = _each_variant(ctx, wl, target, [7, 0])
+    assert_parity(yuv, O.synthesize(wl.inputs, wl.planes, target, 5.0))
+
+
 @pytest.mark.parametrize("precision", [1.0, 1.5])
 @pytest.mark.parametrize("erp_out", [False, True], ids=["persp_out", "erp_out"])
 @pytest.mark.parametrize("inputs", ["erp", "mixed"])
