@@ -67,6 +67,7 @@ struct DevTarget {
     int out_w, out_h;
     float uv_sx, uv_sy;                   // raster size / output size (float)
     float precision;
+    int small;                            // candidate pixels above which a triangle is a large one
     int rs_area;                          // the resize is an exact 2x reduction (area mean)
     double rs_scale_x, rs_scale_y;        // raster size / output size (double), bilinear
     int n_views;

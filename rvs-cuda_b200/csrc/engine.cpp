@@ -186,6 +186,51 @@ int BatchCore::stage_times(float* ms, int max_stages) const {
     return n;
 }
 
+namespace {
+
+// Pixels per radian at the centre of a camera: the focal length of a
+// perspective camera, the width over the horizontal range of an
+// equirectangular one.
+float pixels_per_radian(const rvsb_camera& c) {
+    if (c.projection == RVSB_PROJ_EQUIRECTANGULAR) {
+        const float range = (c.hor_range[1] - c.hor_range[0]) * (3.14159265f / 180.f);
+        return range > 0.f ? (float)c.width / range : 0.f;
+    }
+    return c.focal[0];
+}
+
+// Magnification of a synthesis: output pixels per radian at the raster size
+// over the densest input's.  An equirectangular output stretches its rows by
+// 1 / cos(latitude), sqrt(2) at the median row, which its m includes.
+float magnification(const SlotRequest& r) {
+    float in = 0.f;
+    for (const rvsb_camera& c : r.scene->cams) in = std::max(in, pixels_per_radian(c));
+    const RasterDims rd = raster_dims(r.virt, r.params);
+    float out = pixels_per_radian(r.virt) * (float)rd.w / (float)r.virt.width;
+    if (r.virt.projection == RVSB_PROJ_EQUIRECTANGULAR) out *= 1.41421356f;
+    return in > 0.f ? out / in : 0.f;
+}
+// Above it the ordinary triangles have more than the 4 candidates of the
+// unmagnified threshold.
+constexpr float kMagnified = 1.1f;
+
+// Candidate pixels up to which a magnified view's triangles stay with their
+// lanes.  An input pixel spacing seen m times magnified gives candidate boxes
+// of about m + 1 pixels a side, somewhat more where the surface is slanted.  A
+// threshold below that lists nearly every triangle, which overflows the list:
+// 3 x ERP 1102x550 into ERP 3890x1944 (m = 5) 1303 us with 16, 724 with 49; 2 x
+// 480x270 into 1920x1080 (m = 4) 211 with 16, 146 with 25, 149 with 36; 4 x
+// 240x136 (m = 8) 509 with 64, 244 with 100.  One far above it leaves stretched
+// triangles to single lanes: m = 2, 193 us with 9 and 16, 211 with 36, 270 with
+// 120.  Below 16 nothing is gained (m = 1.5, 224 us with 4 to 16).
+int magnified_threshold(float m) {
+    if (!(m > kMagnified)) return 4;
+    const int side = (int)std::min(20.f, std::max(4.f, std::ceil(m + 1.2f)));
+    return side * side;
+}
+
+}  // namespace
+
 void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape& sh) {
     std::memset(&T, 0, sizeof(T));
     const rvsb_scene* sc = r.scene;
@@ -241,6 +286,8 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     D.out_w = virt.width;
     D.out_h = virt.height;
     D.precision = p.precision;
+    D.small = kRasterVariants[sh.variant].small;
+    if (D.small == 0) D.small = magnified_threshold(magnification(r));
     if (rd.rescale) {
         D.rescale = 1;
         D.uv_sx = (float)rd.w / (float)virt.width;
@@ -341,56 +388,6 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     }
 }
 
-namespace {
-
-// Pixels per radian at the centre of a camera: the focal length of a
-// perspective camera, the width over the horizontal range of an
-// equirectangular one.
-float pixels_per_radian(const rvsb_camera& c) {
-    if (c.projection == RVSB_PROJ_EQUIRECTANGULAR) {
-        const float range = (c.hor_range[1] - c.hor_range[0]) * (3.14159265f / 180.f);
-        return range > 0.f ? (float)c.width / range : 0.f;
-    }
-    return c.focal[0];
-}
-
-// Largest magnification of a batch: output pixels per radian at the raster size
-// over the densest input's.  An equirectangular output stretches its rows by
-// 1 / cos(latitude), sqrt(2) at the median row, which its m includes.
-float magnification(const SlotRequest* reqs, int n, bool& erp_out) {
-    float m = 0.f;
-    erp_out = false;
-    for (int k = 0; k < n; ++k) {
-        const SlotRequest& r = reqs[k];
-        float in = 0.f;
-        for (const rvsb_camera& c : r.scene->cams) in = std::max(in, pixels_per_radian(c));
-        const RasterDims rd = raster_dims(r.virt, r.params);
-        float out = pixels_per_radian(r.virt) * (float)rd.w / (float)r.virt.width;
-        if (r.virt.projection == RVSB_PROJ_EQUIRECTANGULAR) {
-            out *= 1.41421356f;
-            erp_out = true;
-        }
-        if (in > 0.f) m = std::max(m, out / in);
-    }
-    return m;
-}
-
-// Candidate pixels up to which a magnified view's triangles stay with their
-// lanes.  An input pixel spacing seen m times magnified gives candidate boxes
-// of about m + 1 pixels a side, somewhat more where the surface is slanted.  A
-// threshold below that lists nearly every triangle, which overflows the list:
-// 3 x ERP 1102x550 into ERP 3890x1944 (m = 5) 1303 us with 16, 724 with 49; 2 x
-// 480x270 into 1920x1080 (m = 4) 211 with 16, 146 with 25, 149 with 36; 4 x
-// 240x136 (m = 8) 509 with 64, 244 with 100.  One far above it leaves stretched
-// triangles to single lanes: m = 2, 193 us with 9 and 16, 211 with 36, 270 with
-// 120.  Below 16 nothing is gained (m = 1.5, 224 us with 4 to 16).
-int magnified_threshold(float m) {
-    const int side = (int)std::min(20.f, std::max(4.f, std::ceil(m + 1.2f)));
-    return side * side;
-}
-
-}  // namespace
-
 BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) const {
     BatchShape sh;
     sh.slots = n;
@@ -418,9 +415,6 @@ BatchShape BatchCore::shape_of(const SlotRequest* reqs, int n, int variant) cons
         sh.max_out_h = std::max(sh.max_out_h, r.virt.height);
     }
     sh.inputs = erp ? (persp ? 2 : 1) : 0;
-    bool erp_out;
-    sh.small = kRasterVariants[variant].small;
-    if (sh.small == 0) sh.small = magnified_threshold(magnification(reqs, n, erp_out));
     // The four words per pixel that the inpainting scans use later hold the
     // z-buffers of up to four views, or, for more views, of three at a time
     // and half of the running blend (its other half takes the codes').
@@ -449,7 +443,7 @@ int BatchCore::launch_variant(const SlotRequest* reqs, int n, int variant, cudaS
     cur_ ^= 1;
     const TablePtr tabs{tables_.as<SlotTable>()};
     if (use_graphs_ && !profiling_) {
-        const std::vector<int> key = {sh.slots, sh.variant, sh.small, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
+        const std::vector<int> key = {sh.slots, sh.variant, sh.vg, sh.max_views, sh.max_w, sh.max_h, sh.max_wo,
                                       sh.max_ho, sh.aux, sh.ms, sh.extras, sh.erp_out, sh.int_pow, sh.inputs, sh.rescale, sh.max_out_w, sh.max_out_h};
         auto it = graphs_.find(key);
         if (it == graphs_.end()) {
@@ -492,9 +486,13 @@ constexpr int kBatchVariant = 1;
 constexpr int kBatchVariantMinSlots = 8;
 
 int default_variant(const SlotRequest* reqs, int n) {
-    bool erp_out;
-    const float m = magnification(reqs, n, erp_out);
-    if (m > 1.1f) return kMagnifiedVariant;
+    float m = 0.f;
+    bool erp_out = false;
+    for (int k = 0; k < n; ++k) {
+        m = std::max(m, magnification(reqs[k]));
+        if (reqs[k].virt.projection == RVSB_PROJ_EQUIRECTANGULAR) erp_out = true;
+    }
+    if (m > kMagnified) return kMagnifiedVariant;
     if (!erp_out && m <= 0.6f) return kMinifiedVariant;
     return n >= kBatchVariantMinSlots ? kBatchVariant : kDefaultVariant;
 }

@@ -13,7 +13,6 @@ namespace rvsb {
 struct BatchShape {
     int slots = 0;
     int variant = 0;         // raster variant (kRasterVariants)
-    int small = 0;           // candidate pixels above which a triangle goes to the list
     int aux = 0;             // some slot wants auxiliary outputs
     int ms = 0;              // some slot blends multispectrally
     int erp_out = 0;         // some output is equirectangular
@@ -77,7 +76,7 @@ int launch_batch(const Tabs& tabs, const BatchShape& shape, cudaStream_t stream,
 
 // Raster variants the autotuner chooses from: quad rows per warp of the mesh
 // kernel (0: by the launch's size) and the candidate pixels above which a
-// triangle goes to the list of large ones (0: by the magnification).  Every variant gives identical
+// triangle goes to the list of large ones (0: by each slot's magnification).  Every variant gives identical
 // results.
 struct RasterVariant {
     int rows, small;

@@ -291,7 +291,7 @@ struct LargeQueue {
 // have one more strip, whose lanes take the seam triangles of one row each.
 template <int kIn, bool kErpOut, bool kScaled, class Tabs>
 __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_constant__ Tabs tabs, int g0, int gv,
-                                                                   int rows, int small) {
+                                                                   int rows) {
     __shared__ uint4 s_queue[MESH_WARPS][QUEUE];
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.z / gv);
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
                 t[1].mnx = fminf(nx, dx); t[1].mxx = fmaxf(xx, dx);
                 t[1].mny = fminf(ny, dy); t[1].mxy = fmaxf(xy, dy);
                 t[1].m2 = fmaxf(md, fmaxf(sq2(t[1].a0c0, t[1].c1a1), sq2(__fsub_rn(dx, c.x), __fsub_rn(dy, c.y))));
-                raster_small(o, t, tri, small);
+                raster_small(o, t, tri, T.small);
                 if (__any_sync(0xffffffffu, t[0].large || t[1].large)) {
                     queue.push(tab.b, lane, t[0].large, tri, view, t[0].wide, t[0].box);
                     queue.push(tab.b, lane, t[1].large, tri + 1u, view, t[1].wide, t[1].box);
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(32 * MESH_WARPS, 8) mesh_kernel(const __grid_c
             s[0].mny = fminf(fminf(A.y, B.y), C.y); s[0].mxy = fmaxf(fmaxf(A.y, B.y), C.y);
             s[0].m2 = fmaxf(sq2(s[0].c0b0, s[0].b1c1), fmaxf(sq2(s[0].a0c0, s[0].c1a1),
                                                              sq2(__fsub_rn(A.x, B.x), __fsub_rn(A.y, B.y))));
-            raster_small(o, s, tri + (uint32_t)t, small);
+            raster_small(o, s, tri + (uint32_t)t, T.small);
             queue.push(tab.b, lane, s[0].large, tri + (uint32_t)t, view, s[0].wide, s[0].box);
         }
     }
@@ -755,8 +755,7 @@ static void launch_mesh_kernel(const Tabs& tabs, const BatchShape& sh, int g0, i
     const int fixed = kRasterVariants[sh.variant].rows, rows = fixed ? fixed : rows_per_warp(sh, gv);
     const int strips = (sh.max_w - 1 + STRIP - 1) / STRIP + (kErpOut ? 1 : 0);  // and the seam's
     const dim3 grid((strips + MESH_WARPS - 1) / MESH_WARPS, (sh.max_h - 1 + rows - 1) / rows, sh.slots * gv);
-    launch_dependent(mesh_kernel<kIn, kErpOut, kScaled, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rows,
-                     sh.small);
+    launch_dependent(mesh_kernel<kIn, kErpOut, kScaled, Tabs>, grid, dim3(32 * MESH_WARPS), 0, s, tabs, g0, gv, rows);
 }
 
 // The kernel instantiated for what the launch holds (without the projections
