@@ -581,6 +581,8 @@ rvsb_status rvsb_synthesize_host(rvsb_context* ctx, const rvsb_camera* inputs, i
         ctx->host_scene = sc;
     }
     return guarded(ctx, [&]() -> rvsb_status {
+        // Before the first allocation: another device may be current.
+        check(cudaSetDevice(ctx->device), "cudaSetDevice");
         for (int v = 0; v < n_inputs; ++v)
             if (!host_planes[v].y || !host_planes[v].u || !host_planes[v].v || !host_planes[v].depth)
                 throw ArgError("null plane");
@@ -611,7 +613,6 @@ rvsb_status rvsb_synthesize_host(rvsb_context* ctx, const rvsb_camera* inputs, i
         // view's colour is decoded as it arrives.  4 x 1920x1080 (41.5 MB up):
         // 1374 -> 1125 us a call, of which the link takes 870.
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        check(cudaSetDevice(ctx->device), "cudaSetDevice");
         if (!ctx->host_copy) check(cudaStreamCreateWithFlags(&ctx->host_copy, cudaStreamNonBlocking), "cudaStreamCreate");
         if (!ctx->host_ready)
             check(cudaEventCreateWithFlags(&ctx->host_ready, cudaEventDisableTiming), "cudaEventCreate");
