@@ -295,7 +295,8 @@ rvsb_status rvsb_create(int device, size_t hbm_budget_bytes, rvsb_context** out)
 void rvsb_destroy(rvsb_context* ctx) {
     if (!ctx) return;
     if (ctx->host_scene) rvsb_scene_destroy(ctx->host_scene);
-    cudaSetDevice(ctx->device);
+    // Contexts that made no host call leave the current device alone.
+    if (ctx->host_out || ctx->host_copy || ctx->host_ready) cudaSetDevice(ctx->device);
     if (ctx->host_out) cudaFree(ctx->host_out);
     if (ctx->host_copy) cudaStreamDestroy(ctx->host_copy);
     if (ctx->host_ready) cudaEventDestroy(ctx->host_ready);

@@ -1,6 +1,6 @@
 """rvsb_synthesize_host and the caller's current device, on a fake runtime with
 two devices: what the call allocates lies on its context's device, whichever
-is current."""
+is current, and a context without such calls never changes it when it goes."""
 import numpy as np
 import pytest
 
@@ -42,3 +42,10 @@ def test_output_staging_on_the_contexts_device(fake):
     _host_call(ctx, cams, 64, 32)
     assert [(f.device, f.out_device) for f in fake.launches()] == [(1, 1), (1, 1)]
     ctx.close()
+
+
+def test_destroying_an_idle_context_leaves_the_current_device(fake):
+    ctx = rvsb.Context(1)
+    fake.lib.fake_set_device(0)
+    ctx.close()
+    assert fake.lib.fake_device() == 0
