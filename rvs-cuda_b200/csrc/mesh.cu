@@ -243,19 +243,27 @@ __device__ __forceinline__ void raster_small(const MeshTarget& o, Tri (&t)[N], u
 // A warp's large triangles on their way to the slot's list: at most 31 wait
 // in the warp's queue in shared memory; full groups of 32 go out together
 // (one atomic on the list's length, coalesced 16-byte stores).
+//
+// A group that passes the list's capacity is dropped: large_kernel sees the
+// length and goes over the whole mesh instead.  The warp enters nothing more
+// after it, so the length, a 32-bit number, stays within 32 entries per warp
+// of the capacity: at most 2^28 input pixels a view, four views a launch and
+// 4 quad rows a warp make 8.7 M warps, 2.8e8 entries, beside a capacity of at
+// most 3.9e8.  (One triangle over much of a large output has thousands of
+// bands, so that counting them all could pass 2^31.)
 struct LargeQueue {
     uint4* q;       // QUEUE entries of this warp
-    int n;
+    int n;          // of them waiting; negative: the list is full
     __device__ void flush(const SlotBuffers& B, int lane, int count) {
         __syncwarp();
         int base = 0;
         if (lane == 0) base = atomicAdd(&B.status->n_large, count);
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (lane < count) {
-            // Past the capacity the entry is dropped; large_kernel sees the
-            // length and goes over the whole mesh instead.
-            if (base + lane < B.large_capacity) B.large[base + lane] = q[lane];
+        if (base > B.large_capacity - count) {
+            n = INT_MIN;
+            return;
         }
+        if (lane < count) B.large[base + lane] = q[lane];
         __syncwarp();
         const uint4 rest = q[32 + lane];
         __syncwarp();
@@ -270,7 +278,7 @@ struct LargeQueue {
         const int band = general ? 1 << 20 : max(1, kEntryPixels / max(1, w));
         int y = b.y;
         unsigned m;
-        while ((m = __ballot_sync(0xffffffffu, push))) {
+        while (n >= 0 && (m = __ballot_sync(0xffffffffu, push))) {
             if (push) {
                 const int ye = min(b.w, y + band - 1);
                 q[n + __popc(m & ((1u << lane) - 1u))] =
