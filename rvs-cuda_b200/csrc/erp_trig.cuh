@@ -70,7 +70,9 @@ __device__ __forceinline__ double sqrt45(double v) {
 __device__ __forceinline__ double atan44(double Y, double X) {
     float rx, rd;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"((float)X));
-    const float k = rintf((float)Y * rx * 64.f);
+    // Held to the table whatever X and Y are (subnormals make rx infinite, a
+    // vanishing root NaN); the caller discards the result of such arguments.
+    const float k = fminf(rintf((float)Y * rx * 64.f), 64.f);
     const double c = (double)(k * 0.015625f);
     const double num = __fma_rn(-c, X, Y), den = __fma_rn(c, Y, X);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rd) : "f"((float)den));

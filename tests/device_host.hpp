@@ -15,6 +15,8 @@
 #include <thread>
 #include <vector>
 
+#define __noinline__ __attribute__((noinline))
+
 using std::max;
 using std::min;
 using std::isfinite;
