@@ -225,27 +225,41 @@ __device__ __forceinline__ bool tri_range(float4 A, float4 B, float4 C, int wo, 
 
 // Candidate x range of row y for a large triangle.  Each edge test
 // n_k = a_k*tx + b_k*ty + c_k >= -1e-6*den (n_3 = den - n_1 - n_2) bounds tx
-// on one side; the bound is widened by 16 ulp of its terms plus 1e-3, and an
-// edge whose bound is not reliable to half a pixel (nearly horizontal edges)
-// is not used.  Turned into pixels it is widened by another 0.01, which covers
-// the rounding of cx - 0.5 + bound (at most 3 roundings of values below 2^16,
-// under 0.004 each where the pixel lies in an image at most 32768 wide).
-// Every pixel of the span is still tested exactly, so the span only has to
-// contain the covered pixels.  (Stretched triangles are thin: widened by a
-// whole pixel on either side, a row of one covered pixel had three
-// candidates or more, and the kernel took twice as long.)
+// on one side.  The span has to contain every pixel the coverage test accepts
+// (each of its pixels is still tested exactly), so the bound is widened by
+// what rounding can add, 16 ulp of the terms that are rounded (u = 2^-24),
+// plus 1e-3:
+//  - The test rounds the two products of n_1 or n_2 and their sum, at most 2u
+//    of their magnitudes; this computation rounds b*ty, the right-hand side
+//    and the quotient, at most 9u of its terms and the bound together.
+//  - n_3 = den * ((1 - l1) - l2) carries the errors of all four products,
+//    which cancel on a long thin triangle: at most 2u of (|a_1| + |a_2|)|tx| +
+//    (|b_1| + |b_2|)|ty| plus 2u of den, and as much again for a_3, b_3 and
+//    the right-hand side, with |tx| at most that of the box's outer columns.
+//    (Taken from a_3 and b_3 alone the bound left out up to 1.7% of the
+//    covered pixels next to a short third edge.)
+// An edge whose bound is not reliable to half a pixel (nearly horizontal
+// edges, the short side opposite a far vertex) is not used.  Turned into
+// pixels the bound is widened by another 0.01, which covers the rounding of
+// the pixel centre's tx and of cx - 0.5 + bound: in an image at most 32768
+// wide below 0.002 each, but for what 16u of a longer bound already holds.
+// (Stretched triangles are thin: widened by a whole pixel on either side, a
+// row of one covered pixel had three candidates or more, and the kernel took
+// twice as long.)
 __device__ __forceinline__ void row_span(const TriSetup& s, float cx, float cy, int y, int& xl, int& xr) {
     const float eps = 1e-6f, u = 5.9604645e-8f;
     const float ty = __fsub_rn(__fadd_rn((float)y, 0.5f), cy);
     const float a[3] = {s.b1c1, s.c1a1, -(s.b1c1 + s.c1a1)};
     const float b[3] = {s.c0b0, s.a0c0, -(s.c0b0 + s.a0c0)};
     const float c[3] = {0.f, 0.f, s.den};
+    const float far_x = fmaxf(fabsf((float)s.x0 + 0.5f - cx), fabsf((float)s.x1 + 0.5f - cx));
+    const float sum = (fabsf(a[0]) + fabsf(a[1])) * far_x + (fabsf(b[0]) + fabsf(b[1])) * fabsf(ty) + fabsf(s.den);
     float lo = -INFINITY, hi = INFINITY;
     bool empty = false;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float rhs = -eps * s.den - b[k] * ty - c[k];
-        const float mag = fabsf(eps * s.den) + fabsf(b[k] * ty) + fabsf(c[k]);
+        const float mag = k == 2 ? sum : fabsf(eps * s.den) + fabsf(b[k] * ty);
         if (a[k] == 0.f) {
             if (rhs > 16.f * u * mag) empty = true;
             continue;
