@@ -1,0 +1,115 @@
+"""Long stretched triangles and full lists of them, against the oracle: per-view
+coverage and hole mask identical, output at the parity bar.  What each scene
+puts into the list of large triangles is counted from the oracle's warped
+vertices, so the scenes are known to reach what they are for."""
+import copy
+
+import numpy as np
+import pytest
+
+import oracle as O
+import rvsb
+from rvsb import scenes
+from helpers import assert_parity, gpu_synthesize
+
+pytestmark = pytest.mark.gpu
+
+THRESHOLD = 4  # candidate pixels of raster variant 0
+BAND = 8192    # pixels of a list entry
+
+
+def _capacity(inputs):
+    return max(1 << 14, sum(c.width * c.height for c in inputs) // 11)
+
+
+def _listed(uv, z, wo, ho):
+    """(entries, bounding-box diagonals) of one view's triangles above the
+    threshold: two per quad, emitted, front-facing, their candidate boxes cut
+    into bands of rows."""
+    x, y = uv[..., 0].astype(np.float64), uv[..., 1].astype(np.float64)
+    ok = (z > 0) & (x > 0)
+    diag = ok[:-1, 1:] & ok[1:, :-1]
+    entries, lengths = 0, []
+    for corner, (a, b, c) in ((ok[:-1, :-1], ((0, 0), (0, 1), (1, 0))), (ok[1:, 1:], ((1, 1), (1, 0), (0, 1)))):
+        at = lambda m, p: m[p[0]:m.shape[0] - 1 + p[0], p[1]:m.shape[1] - 1 + p[1]]
+        ax, bx, cx = (at(x, p) for p in (a, b, c))
+        ay, by, cy = (at(y, p) for p in (a, b, c))
+        den = (by - cy) * (ax - cx) + (cx - bx) * (ay - cy)
+        mnx, mxx = np.minimum(np.minimum(ax, bx), cx), np.maximum(np.maximum(ax, bx), cx)
+        mny, mxy = np.minimum(np.minimum(ay, by), cy), np.maximum(np.maximum(ay, by), cy)
+        w = np.minimum(wo - 1, np.rint(mxx) - 1) - np.maximum(0, np.rint(mnx)) + 1
+        h = np.minimum(ho - 1, np.rint(mxy) - 1) - np.maximum(0, np.rint(mny)) + 1
+        with np.errstate(invalid="ignore"):
+            on = diag & corner & (den > 1e-6) & (w > 0) & (h > 0) & (w * h > THRESHOLD)
+        entries += int(np.ceil(h[on] / np.maximum(1, BAND // w[on])).sum())
+        lengths.append(np.hypot(mxx - mnx, mxy - mny)[on])
+    return entries, np.concatenate(lengths)
+
+
+def _against_oracle(ctx, wl, target, planes):
+    """The synthesis with variant 0 (and, bit for bit, 7) against the oracle;
+    returns the entries of the list and the triangles' lengths."""
+    sc = rvsb.Scene(ctx, wl.inputs)
+    for i, p in enumerate(planes):
+        sc.upload(i, [np.ascontiguousarray(a, np.uint16) for a in p], on_device=False)
+    sc.set_raster_variant(0)
+    yuv, dbg, _ = gpu_synthesize(ctx, wl.inputs, planes, target, 5.0, debug=True, scene=sc)
+    entries, lengths, quality = 0, [], []
+    for v, (cam, (y, u, w, d)) in enumerate(zip(wl.inputs, planes)):
+        uv, vd, wrap = O.warp(cam, target, O.decode_depth(d, cam))
+        n, l = _listed(uv, vd, target.width, target.height)
+        entries += n
+        lengths.append(l)
+        _, _, valid = O.raster(O.decode_color(y, u, w, cam.bit_depth_color), vd, uv, target.width, target.height, wrap)
+        gpu = dbg["view_validity"][v] > 0
+        assert np.array_equal(gpu, valid > 0), f"view {v}: coverage differs at {np.argwhere(gpu != (valid > 0))[:5]}"
+    assert_parity(yuv, O.synthesize(wl.inputs, planes, target, 5.0))
+    sc.set_raster_variant(7)
+    other, _ = gpu_synthesize(ctx, wl.inputs, planes, target, 5.0, scene=sc)
+    for a, b in zip(other, yuv):
+        np.testing.assert_array_equal(a, b)
+    return entries, np.concatenate(lengths)
+
+
+def _scaled(target, w, h):
+    t = copy.deepcopy(target)
+    for i, (new, old) in enumerate(((w, target.width), (h, target.height))):
+        t.focal[i] *= new / old
+        t.principle_point[i] = new / 2.0
+    t.width, t.height = w, h
+    return t
+
+
+@pytest.mark.parametrize("roll", [0.0, 25.0, 60.0])
+def test_depth_steps_stretch_across_the_view(ctx, roll):
+    """Patches of 64 x 48 pixels, near or far, seen from beside: triangles up
+    to several hundred pixels long between them, some with boxes of more than
+    one band, and the list not full."""
+    wl = scenes.random_pose_small(n_views=2, w=512, h=288, seed=340)
+    rng = np.random.default_rng(341)
+    planes = []
+    for y, u, v, d in wl.planes:
+        step = np.kron(rng.integers(0, 2, (6, 8)), np.ones((48, 64), int))
+        planes.append((y, u, v, (step * 40000 + 6000 + d // 64).astype(np.uint16)))
+    target = copy.deepcopy(wl.targets[0])
+    target.position[1] += 0.5
+    target.position[2] += 0.15
+    target.rotation[2] += roll
+    entries, lengths = _against_oracle(ctx, wl, target, planes)
+    bands = entries - len(lengths)
+    assert entries <= _capacity(wl.inputs) and bands > 100 and (lengths > 300).sum() > 500, (
+        entries, bands, lengths.max())
+
+
+@pytest.mark.parametrize("w,h,wo,ho", [(160, 96, 640, 384), (128, 96, 1920, 1080)])
+def test_noise_overflows_the_list(ctx, w, h, wo, ho):
+    """Depth samples of pure noise: nearly every triangle is stretched over
+    much of the view, and their bands are several times what the list
+    holds."""
+    wl = scenes.random_pose_small(n_views=2, w=w, h=h, seed=350)
+    rng = np.random.default_rng(351)
+    planes = [(y, u, v, rng.integers(0, 65536, d.shape).astype(np.uint16)) for y, u, v, d in wl.planes]
+    target = _scaled(wl.targets[0], wo, ho)
+    target.position[1] += 0.2
+    entries, _ = _against_oracle(ctx, wl, target, planes)
+    assert entries > 1.5 * _capacity(wl.inputs), entries
