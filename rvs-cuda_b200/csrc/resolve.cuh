@@ -49,15 +49,17 @@ __device__ __forceinline__ float2 sq_len2(float dx, float dy) {
     return make_float2(hi, __fadd_rn(e, __fadd_rn(ep, eq)));
 }
 
-// tri_quality (device_common.cuh) without double arithmetic: the longest
-// edge is picked by its squared length in float where that decides it, its
-// squared length kept to about 46 bits, and an approximate square root
-// corrected by one Newton step from the remainder, which gives the correctly
-// rounded root except where that lies within about 2^-20 of a rounding
-// boundary (relative to the spacing of floats).  Where edges tie (to 2^-20)
-// or are tiny, the double evaluation runs.  With the colour unpacking and the
-// blend's powers below: 94 -> 86.6 M warp instructions, 123 -> 117 us on 4
-// views of 1920x1080.
+// tri_quality (device_common.cuh) without double arithmetic, the same float:
+// the longest edge is picked by its squared length in float where that decides
+// it, its squared length kept to about 46 bits, and an approximate square root
+// corrected by one Newton step from the remainder.  Root and correction
+// together are within 2^-43 of the root (2^-46 from the square, 2^-45 each
+// from the remainder's rounding and from taking 0.5 * y, 2^-22 off, for half
+// the reciprocal root); the sum is rounded to float with 2^-40 added and taken
+// off, and where the two differ (1 in 2^16 roots), edges tie (to 2^-20) or are
+// tiny, the double evaluation runs.  With the colour unpacking and the blend's
+// powers below: 94 -> 86.6 M warp instructions, 123 -> 117 us on 4 views of
+// 1920x1080.
 __device__ __forceinline__ float tri_quality_fast(float4 A, float4 B, float4 C, float precision) {
     const float bx = __fsub_rn(B.x, C.x), by = __fsub_rn(B.y, C.y);
     const float ax = __fsub_rn(A.x, C.x), ay = __fsub_rn(A.y, C.y);
@@ -65,15 +67,16 @@ __device__ __forceinline__ float tri_quality_fast(float4 A, float4 B, float4 C, 
     const float sb = __fmaf_rn(bx, bx, __fmul_rn(by, by)), sa = __fmaf_rn(ax, ax, __fmul_rn(ay, ay)),
                 sd = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
     const float ad = fmaxf(sa, sd), m = fmaxf(sb, ad), second = fmaxf(fminf(sa, sd), fminf(sb, ad));
-    if (!(m > 1e-12f) || second >= __fmul_rn(m, 0.999999f))
-        return tri_quality(A.x, A.y, B.x, B.y, C.x, C.y, precision);
     const bool is_b = sb == m, is_a = sa == m;
     const float2 l = sq_len2(is_b ? bx : is_a ? ax : dx, is_b ? by : is_a ? ay : dy);
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(l.x));
     const float s = __fmul_rn(l.x, y);
     const float rem = __fadd_rn(__fmaf_rn(-s, s, l.x), l.y);
-    float stretch = __fmaf_rn(rem, __fmul_rn(0.5f, y), s);
+    const float c = __fmul_rn(rem, __fmul_rn(0.5f, y)), err = __fmul_rn(s, 9.094947e-13f);  // 2^-40
+    float stretch = __fadd_rn(s, __fadd_rn(c, err));
+    if (!(m > 1e-12f) || second >= __fmul_rn(m, 0.999999f) || stretch != __fadd_rn(s, __fsub_rn(c, err)))
+        return tri_quality(A.x, A.y, B.x, B.y, C.x, C.y, precision);
     if (precision != 1.f) stretch = __fdiv_rn(stretch, precision);  // stretch /= g_rescale
     return fminf(10000.f, fmaxf(1.f, __fsub_rn(10000.f, __fmul_rn(1000.f, stretch))));
 }
