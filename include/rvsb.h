@@ -413,10 +413,10 @@ rvsb_status rvsb_batch_reserve(rvsb_batch* batch, int max_width, int max_height)
 /* Capture each batch shape into a CUDA graph and replay it (default off). */
 rvsb_status rvsb_batch_set_graphs(rvsb_batch* batch, int enable);
 /* Raster autotuner (default off): the first batch of each new shape (batch
- * size bucket, largest input set and output, projections) is run once with
- * every raster variant -- quad rows per warp and the candidate-pixel count
- * above which a triangle is rasterised by a whole warp instead of one lane --
- * and the fastest is kept for that shape.
+ * size bucket, largest input set and output, projections, magnification) is
+ * run once with every raster variant -- quad rows per warp and the
+ * candidate-pixel count above which a triangle is rasterised by a whole warp
+ * instead of one lane -- and the fastest is kept for that shape.
  * All variants give identical outputs. */
 rvsb_status rvsb_batch_set_autotune(rvsb_batch* batch, int enable);
 /* Use one raster variant (0 .. 7) for every call, or -1 for the default or

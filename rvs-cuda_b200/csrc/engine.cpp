@@ -2,6 +2,7 @@
 #include "engine.hpp"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 
@@ -565,16 +566,21 @@ int BatchCore::run(const SlotRequest* reqs, int n, cudaStream_t s, const std::fu
         variant = forced_variant_;
     } else if (autotune_) {
         // The shape the tuner keys on: the batch size bucket and, over the
-        // batch, the largest input set and output and the projections.
+        // batch, the largest input set and output, the projections and the
+        // magnified thresholds (a fixed threshold that suits unmagnified
+        // triangles lists nearly every magnified one).
         const BatchShape sh = shape_of(reqs, n, 0);
-        int proj_in = 0, proj_out = 0;
+        int proj_in = 0, proj_out = 0, small_lo = INT_MAX, small_hi = 0;
         for (int k = 0; k < n; ++k) {
             proj_in |= 1 << reqs[k].scene->cams[0].projection;
             proj_out |= 1 << reqs[k].virt.projection;
+            const int small = magnified_threshold(magnification(reqs[k]));
+            small_lo = std::min(small_lo, small);
+            small_hi = std::max(small_hi, small);
         }
         const int bucket = n == 1 ? 1 : n <= 4 ? 4 : n <= 16 ? 16 : 64;
         const std::vector<int> sig = {bucket, sh.max_views, sh.max_w, sh.max_h, sh.max_wo, sh.max_ho,
-                                      proj_in, proj_out, sh.max_out_w, sh.max_out_h};
+                                      proj_in, proj_out, sh.max_out_w, sh.max_out_h, small_lo, small_hi};
         auto it = tuned_.find(sig);
         if (it == tuned_.end()) it = tuned_.emplace(sig, tune(reqs, n, s)).first;
         variant = it->second;
