@@ -512,11 +512,27 @@ int BatchCore::tune(const SlotRequest* reqs, int n, cudaStream_t s) {
     // percent apart, and among variants within the noise of each other the
     // pick would otherwise be arbitrary (measured: a 1.7% slower one picked
     // for the plain 1080p view).
+    // Variants whose launch is that of an earlier one (same rows, and the same
+    // threshold in every slot) take its time.
     constexpr int kRounds = 5;
-    for (int v = 0; v < NUM_RASTER_VARIANTS; ++v) launch_variant(reqs, n, v, s);
+    bool magnified = false;
+    for (int k = 0; k < n; ++k) magnified = magnified || magnified_threshold(magnification(reqs[k])) != 4;
+    int same[NUM_RASTER_VARIANTS];
+    std::vector<int> timed;
+    for (int v = 0; v < NUM_RASTER_VARIANTS; ++v) {
+        auto small_of = [&](int w) {
+            const int small = kRasterVariants[w].small;
+            return small == 0 && !magnified ? 4 : small;
+        };
+        same[v] = v;
+        for (int u : timed)
+            if (kRasterVariants[u].rows == kRasterVariants[v].rows && small_of(u) == small_of(v)) same[v] = u;
+        if (same[v] == v) timed.push_back(v);
+    }
+    for (int v : timed) launch_variant(reqs, n, v, s);
     float t[NUM_RASTER_VARIANTS][kRounds];
     for (int r = 0; r < kRounds; ++r)
-        for (int v = 0; v < NUM_RASTER_VARIANTS; ++v) {
+        for (int v : timed) {
             check(cudaEventRecord(tune_ev_[0], s), "record");
             launch_variant(reqs, n, v, s);
             check(cudaEventRecord(tune_ev_[1], s), "record");
@@ -525,7 +541,7 @@ int BatchCore::tune(const SlotRequest* reqs, int n, cudaStream_t s) {
         }
     int best = 0;
     float best_ms = 0.f, med[NUM_RASTER_VARIANTS];
-    for (int v = 0; v < NUM_RASTER_VARIANTS; ++v) {
+    for (int v : timed) {
         std::sort(t[v], t[v] + kRounds);
         med[v] = t[v][kRounds / 2];
         if (v == 0 || med[v] < best_ms) {
@@ -534,7 +550,7 @@ int BatchCore::tune(const SlotRequest* reqs, int n, cudaStream_t s) {
         }
     }
     const int fallback = default_variant(reqs, n);
-    if (best_ms > 0.98f * med[fallback]) best = fallback;
+    if (best_ms > 0.98f * med[same[fallback]]) best = fallback;
     use_graphs_ = graphs;
     profiling_ = prof;
     return best;

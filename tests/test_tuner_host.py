@@ -53,3 +53,13 @@ def test_a_choice_is_kept_per_magnification(fake):
     assert fake.lib.fake_launches() == count + 2  # both known by now
     mixed = _run(fake, batch, [1.0, 5.0])
     assert mixed.variant == 7 and fake.lib.fake_launches() > count + 3
+
+
+@pytest.mark.parametrize("zoom,distinct", [(1.0, 5), (5.0, 6)])
+def test_variants_of_the_same_content_are_timed_once(fake, zoom, distinct):
+    """Variants 1, 2 and 4 run the same launch, and 7 too unless the view is
+    magnified: a warm-up and five rounds of the distinct ones, and the call."""
+    batch = _batch(2)
+    batch.set_autotune(True)
+    _run(fake, batch, [zoom, zoom])
+    assert fake.lib.fake_launches() == 6 * distinct + 1
