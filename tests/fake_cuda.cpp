@@ -29,6 +29,7 @@ struct Block {
 };
 std::mutex g_mu;
 std::map<char*, Block> g_blocks;
+std::map<cudaStream_t, int> g_pending;  // copies issued since the stream was last waited for
 std::string g_fail_call;
 int g_fail_after = -1;
 
@@ -71,12 +72,19 @@ void fake_reset() {
     std::lock_guard<std::mutex> lock(g_mu);
     g_launches.clear();
     g_decodes = 0;
+    g_pending.clear();
     g_fail_after = -1;
 }
 void fake_fail(const char* call, int after) {
     std::lock_guard<std::mutex> lock(g_mu);
     g_fail_call = call;
     g_fail_after = after;
+}
+int fake_pending_copies() {
+    std::lock_guard<std::mutex> lock(g_mu);
+    int n = 0;
+    for (const auto& p : g_pending) n += p.second;
+    return n;
 }
 int fake_launches() { return (int)g_launches.size(); }
 void fake_launch(int k, FakeLaunch* out) { *out = g_launches[k]; }
@@ -119,9 +127,12 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
     std::memcpy(d, s, n);
     return result("cudaMemcpy");
 }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t stream) {
     const cudaError_t e = result("cudaMemcpyAsync");
-    if (e == cudaSuccess) std::memcpy(d, s, n);
+    if (e != cudaSuccess) return e;
+    std::memcpy(d, s, n);
+    std::lock_guard<std::mutex> lock(g_mu);
+    ++g_pending[stream];
     return e;
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
@@ -132,7 +143,12 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
     std::free(s);
     return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return result("cudaStreamSynchronize"); }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    const cudaError_t e = result("cudaStreamSynchronize");
+    std::lock_guard<std::mutex> lock(g_mu);
+    g_pending[s] = 0;
+    return e;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return result("cudaStreamWaitEvent"); }
 cudaError_t cudaEventCreate(cudaEvent_t* e) {
     *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));
