@@ -701,14 +701,21 @@ __global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_co
     const bool wrap = T.wrap != 0;
     for (int view = g0; view < min(T.n_views, g0 + gv); ++view) {
         const DevView& V = tab.v[view];
-        const int groups = (V.w - 1 + 31) / 32;
+        // Quads a warp takes at once: 32, fewer where that leaves some warps
+        // without any, since the listed triangles lie together (a row of quads
+        // across a depth step): 160x90 noise magnified 12 times 698 -> 285
+        // us, 6 x 480x270 with bars of 6 rows 1177 -> 688.  Four groups for
+        // every warp: 289 and 436, but 2 x 480x270 noise into ERP 198 -> 262.
+        int per = 32;
+        while (per > 4 && (long long)((V.w - 1 + per - 1) / per) * (V.h - 1) < nw) per /= 2;
+        const int groups = (V.w - 1 + per - 1) / per;
         for (long long g = wid; g < (long long)groups * (V.h - 1); g += nw) {
-            const int i = (int)(g / groups), j0 = (int)(g % groups) * 32, j = j0 + lane;
+            const int i = (int)(g / groups), j0 = (int)(g % groups) * per, j = j0 + lane;
             if (T.cull && V.erp_cone && tile_culled(V, T, j0 / WARP_TILE, i / WARP_TILE)) continue;
             for (int t = 0; t < (wrap ? 4 : 2); ++t) {
                 const uint32_t tri = ((((uint32_t)i << (V.tri_shift - 2)) | (uint32_t)j) << 2) | (uint32_t)t;
                 Large r = {};
-                bool on = j < V.w - 1 && (t < 2 || j == 0);
+                bool on = lane < per && j < V.w - 1 && (t < 2 || j == 0);
                 if (on) {
                     // Emission tests of transform.cpp:161-167.
                     const float4 v01 = __ldg(V.vert + (size_t)i * V.w + j + 1);

@@ -101,11 +101,11 @@ def test_depth_steps_stretch_across_the_view(ctx, roll):
         entries, bands, lengths.max())
 
 
-@pytest.mark.parametrize("w,h,wo,ho", [(160, 96, 640, 384), (128, 96, 1920, 1080)])
+@pytest.mark.parametrize("w,h,wo,ho", [(160, 96, 640, 384), (128, 96, 1920, 1080), (320, 160, 640, 384), (482, 270, 960, 540)])
 def test_noise_overflows_the_list(ctx, w, h, wo, ho):
     """Depth samples of pure noise: nearly every triangle is stretched over
-    much of the view, and their bands are several times what the list
-    holds."""
+    much of the view, and there are more of them than the list holds.  The
+    pass over the whole mesh takes 4, 4, 8 and 16 quads a warp."""
     wl = scenes.random_pose_small(n_views=2, w=w, h=h, seed=350)
     rng = np.random.default_rng(351)
     planes = [(y, u, v, rng.integers(0, 65536, d.shape).astype(np.uint16)) for y, u, v, d in wl.planes]
