@@ -68,10 +68,10 @@ SlotNeeds needs_of(const rvsb_scene* sc, int wo, int ho) {
     SlotNeeds n{};
     for (const auto& c : sc->cams) n.vert += (size_t)c.width * c.height;
     n.out = (size_t)wo * ho;
-    // About 1% of the triangles of an unmagnified view are large; when they
-    // do not fit, large_kernel goes over the whole mesh.
     n.hole_words = (size_t)((wo + 31) / 32) * ho;
     n.sum_words = inpaint_sum_words(wo, ho);
+    // About 1% of the triangles of an unmagnified view are large; when they
+    // do not fit, large_kernel goes over the whole mesh.
     n.large = std::min<size_t>(INT32_MAX / 2, std::max<size_t>(1 << 14, n.vert / 11));
     return n;
 }
@@ -84,59 +84,41 @@ size_t SlotWorkspace::bytes_for(const rvsb_scene* sc, int wo, int ho, bool resca
            n.hole_words * sizeof(uint32_t) + n.sum_words * sizeof(uint64_t) + (rescale ? n.out * (sizeof(float4) + 2 * sizeof(int32_t)) : 0);
 }
 
+// Grows `m` to at least n bytes.  What it holds is its allocation's own size, so
+// that a buffer whose growth failed counts as empty in the calls that follow.
+static void grow(rvsb_context* ctx, DevMem& m, size_t n) {
+    if (m.bytes < n) m.alloc(ctx, n);
+}
+
 void SlotWorkspace::ensure_rescale(rvsb_context* ctx, int wo, int ho) {
     const size_t n = (size_t)wo * ho;
-    if (n > cap_rescale) {
-        pcolor.alloc(ctx, n * sizeof(float4));
-        psrc.alloc(ctx, n * 2 * sizeof(int32_t));
-        cap_rescale = n;
-    }
+    grow(ctx, pcolor, n * sizeof(float4));
+    grow(ctx, psrc, n * 2 * sizeof(int32_t));
 }
 
 void SlotWorkspace::ensure(rvsb_context* ctx, const rvsb_scene* sc, int wo, int ho) {
     const SlotNeeds n = needs_of(sc, wo, ho);
-    if (!status.ptr) status.alloc(ctx, sizeof(DevStatus));
-    if (n.vert > cap_vert) {
-        vert.alloc(ctx, n.vert * sizeof(float4));
-        cap_vert = n.vert;
-    }
-    if (n.large > cap_large) {
-        large.alloc(ctx, n.large * sizeof(uint4));
-        cap_large = n.large;
-    }
-    if (n.hole_words > cap_hole_words) {
-        holes.alloc(ctx, n.hole_words * sizeof(uint32_t));
-        cap_hole_words = n.hole_words;
-    }
-    if (n.sum_words > cap_sum_words) {
-        inpaint_sum.alloc(ctx, n.sum_words * sizeof(uint64_t));
-        cap_sum_words = n.sum_words;
-    }
-    if (n.out > cap_out) {
-        codes.alloc(ctx, n.out * sizeof(uint64_t));
-        scan.alloc(ctx, 4 * n.out * sizeof(uint64_t));
-        cap_out = n.out;
-    }
+    grow(ctx, status, sizeof(DevStatus));
+    grow(ctx, vert, n.vert * sizeof(float4));
+    grow(ctx, large, n.large * sizeof(uint4));
+    grow(ctx, holes, n.hole_words * sizeof(uint32_t));
+    grow(ctx, inpaint_sum, n.sum_words * sizeof(uint64_t));
+    grow(ctx, codes, n.out * sizeof(uint64_t));
+    grow(ctx, scan, 4 * n.out * sizeof(uint64_t));
 }
 
 void SlotWorkspace::ensure_aux(rvsb_context* ctx, int wo, int ho) {
     const size_t n = (size_t)wo * ho;
-    if (n > cap_aux) {
-        aux_depth.alloc(ctx, n * sizeof(float));
-        aux_valid.alloc(ctx, n * sizeof(float));
-        cap_aux = n;
-    }
+    grow(ctx, aux_depth, n * sizeof(float));
+    grow(ctx, aux_valid, n * sizeof(float));
 }
 
 void SlotWorkspace::ensure_ms(rvsb_context* ctx, int n_views, int wo, int ho) {
     const size_t n = (size_t)n_views * wo * ho;
-    if (n > cap_ms) {
-        ms_view.alloc(ctx, n * sizeof(float4));
-        ms_hsum.alloc(ctx, n * sizeof(double));
-        ms_hcnt.alloc(ctx, n * sizeof(int));
-        ms_blur.alloc(ctx, n * sizeof(float));
-        cap_ms = n;
-    }
+    grow(ctx, ms_view, n * sizeof(float4));
+    grow(ctx, ms_hsum, n * sizeof(double));
+    grow(ctx, ms_hcnt, n * sizeof(int));
+    grow(ctx, ms_blur, n * sizeof(float));
 }
 
 BatchCore::BatchCore(rvsb_context* ctx, int slots) : ctx_(ctx), slots_(slots) {
@@ -356,7 +338,7 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     SlotBuffers& B = T.b;
     B.status = ws.status.as<DevStatus>();
     B.large = ws.large.as<uint4>();
-    B.large_capacity = (int)ws.cap_large;
+    B.large_capacity = (int)std::min<size_t>(INT32_MAX / 2, ws.large.bytes / sizeof(uint4));
     B.codes = ws.codes.as<uint64_t>();
     B.holes = ws.holes.as<uint32_t>();
     for (int s = 0; s < 4; ++s) B.scan[s] = ws.scan.as<uint64_t>() + (size_t)s * npix;

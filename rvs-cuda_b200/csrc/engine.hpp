@@ -88,12 +88,9 @@ struct SlotWorkspace {
     DevMem aux_depth, aux_valid;  // blended depth / validity (auxiliary outputs only)
     DevMem inpaint_sum;           // column minima of the inpainting's row groups
     DevMem ms_view, ms_hsum, ms_hcnt, ms_blur;  // multispectral blending only
-    size_t cap_ms = 0;            // view-pixels the multispectral buffers hold
     void ensure_ms(rvsb_context* ctx, int n_views, int wo, int ho);
     DevMem pcolor, psrc;          // Precision != 1: raster-size colour and inpainting sources
-    size_t cap_rescale = 0;
     void ensure_rescale(rvsb_context* ctx, int wo, int ho);
-    size_t cap_vert = 0, cap_out = 0, cap_large = 0, cap_aux = 0, cap_hole_words = 0, cap_sum_words = 0;
     void ensure_aux(rvsb_context* ctx, int wo, int ho);
 
     // Bytes a slot needs for `scene` at raster size wo x ho (rescale: plus

@@ -40,6 +40,14 @@ const Block* block_of(const void* p) {
     return static_cast<const char*>(p) < it->first + it->second.bytes ? &it->second : nullptr;
 }
 
+// Whether `bytes` from `p` on lie in one allocation.
+bool backed(const void* p, size_t bytes) {
+    auto it = g_blocks.upper_bound(const_cast<char*>(static_cast<const char*>(p)));
+    if (it == g_blocks.begin()) return false;
+    --it;
+    return static_cast<const char*>(p) + bytes <= it->first + it->second.bytes;
+}
+
 // The error of the call `name` where the test asked for one.
 cudaError_t result(const char* name) {
     std::lock_guard<std::mutex> lock(g_mu);
@@ -55,6 +63,7 @@ extern "C" {
 struct FakeLaunch {
     int device, out_device, slots, variant, small, views, decodes_before, decodes_at_resolve;
     float precision;
+    int unbacked;  // workspace buffers without an allocation of their size behind them
 };
 
 }  // extern "C"
@@ -197,6 +206,41 @@ rvsb_status rvsb_inpaint_sources_noalloc(const uint8_t*, int, int, int32_t*, voi
 
 namespace rvsb {
 
+size_t inpaint_sum_words(int wo, int ho) { return (size_t)3 * ((ho + 31) / 32) * wo; }
+
+// What the kernels of a slot write beside its outputs.
+static int unbacked_buffers(const SlotTable& t) {
+    const size_t n = (size_t)t.t.wo * t.t.ho;
+    int bad = 0;
+    auto need = [&](const void* p, size_t bytes) { bad += !backed(p, bytes); };
+    need(t.b.status, sizeof(DevStatus));
+    need(t.b.large, sizeof(uint4) * (size_t)t.b.large_capacity);
+    need(t.b.codes, 8 * n);
+    need(t.b.holes, 4 * (size_t)((t.t.wo + 31) / 32) * t.t.ho);
+    for (const uint64_t* p : t.b.scan) need(p, 8 * n);
+    need(t.b.inpaint_sum, 8 * inpaint_sum_words(t.t.wo, t.t.ho));
+    for (int v = 0; v < t.t.n_views; ++v) {
+        need(t.v[v].vert, sizeof(float4) * (size_t)t.v[v].w * t.v[v].h);
+        need(t.v[v].z, 8 * n);
+    }
+    if (t.t.rescale) {
+        need(t.b.pcolor, sizeof(float4) * n);
+        need(t.b.psrc, 8 * n);
+    }
+    if (t.aux.on) {
+        need(t.aux.acc_depth, 4 * n);
+        need(t.aux.acc_valid, 4 * n);
+    }
+    if (t.ms.on) {
+        need(t.ms.yq, 8 * n * t.t.n_views);
+        need(t.ms.uv, 8 * n * t.t.n_views);
+        need(t.ms.hsum, 8 * n * t.t.n_views);
+        need(t.ms.hcnt, 4 * n * t.t.n_views);
+        need(t.ms.blur, 4 * n * t.t.n_views);
+    }
+    return bad;
+}
+
 template <class Tabs>
 int launch_batch(const Tabs& tabs, const BatchShape& sh, cudaStream_t, cudaEvent_t*,
                  const std::function<void()>& before_resolve) {
@@ -210,6 +254,7 @@ int launch_batch(const Tabs& tabs, const BatchShape& sh, cudaStream_t, cudaEvent
     f.small = t.t.small;
     f.views = t.t.n_views;
     f.precision = t.t.precision;
+    for (int k = 0; k < sh.slots; ++k) f.unbacked += unbacked_buffers(tabs.at(k));
     f.decodes_before = g_decodes;
     if (before_resolve) before_resolve();
     f.decodes_at_resolve = g_decodes;
@@ -221,7 +266,6 @@ template int launch_batch<TableParam>(const TableParam&, const BatchShape&, cuda
 template int launch_batch<TablePtr>(const TablePtr&, const BatchShape&, cudaStream_t, cudaEvent_t*,
                                     const std::function<void()>&);
 
-size_t inpaint_sum_words(int wo, int ho) { return (size_t)3 * ((ho + 31) / 32) * wo; }
 void launch_decode_color(const uint16_t*, const uint16_t*, const uint16_t*, int, int, uint64_t*, cudaStream_t) {
     ++g_decodes;
 }

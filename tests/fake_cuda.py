@@ -13,11 +13,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 
 class Launch(ctypes.Structure):
     """FakeLaunch: the current device and that of the output planes, what the
-    launch's first slot holds, and the colour decodes issued before the launch
-    and before its resolve."""
+    launch's first slot holds, the colour decodes issued before the launch and
+    before its resolve, and the workspace buffers of its slots that have no
+    allocation of their size behind them."""
 
     _fields_ = [(n, ctypes.c_int) for n in ("device", "out_device", "slots", "variant", "small", "views",
-                                            "decodes_before", "decodes_at_resolve")] + [("precision", ctypes.c_float)]
+                                            "decodes_before", "decodes_at_resolve")] + [("precision", ctypes.c_float),
+                                                                                            ("unbacked", ctypes.c_int)]
 
 
 def build(out_dir):
