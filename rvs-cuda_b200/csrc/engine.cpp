@@ -197,18 +197,42 @@ float magnification(const SlotRequest& r) {
 // unmagnified threshold.
 constexpr float kMagnified = 1.1f;
 
-// Candidate pixels up to which a magnified view's triangles stay with their
-// lanes.  An input pixel spacing seen m times magnified gives candidate boxes
-// of about m + 1 pixels a side, somewhat more where the surface is slanted.  A
-// threshold below that lists nearly every triangle, which overflows the list:
-// 3 x ERP 1102x550 into ERP 3890x1944 (m = 5) 1303 us with 16, 724 with 49; 2 x
-// 480x270 into 1920x1080 (m = 4) 211 with 16, 146 with 25, 149 with 36; 4 x
-// 240x136 (m = 8) 509 with 64, 244 with 100.  One far above it leaves stretched
-// triangles to single lanes: m = 2, 193 us with 9 and 16, 211 with 36, 270 with
-// 120.  Below 16 nothing is gained (m = 1.5, 224 us with 4 to 16).
-int magnified_threshold(float m) {
-    if (!(m > kMagnified)) return 4;
-    const int side = (int)std::min(20.f, std::max(4.f, std::ceil(m + 1.2f)));
+// Candidate pixels up to which a view's triangles stay with their lanes.  An
+// input pixel spacing seen m times magnified gives candidate boxes of about m + 1
+// pixels a side, somewhat more where the surface is slanted.  A threshold below
+// that lists nearly every triangle, which overflows the list: 3 x ERP 1102x550
+// into ERP 3890x1944 (m = 5) 1303 us with 16, 724 with 49; 2 x 480x270 into
+// 1920x1080 (m = 4) 211 with 16, 146 with 25, 149 with 36.  One far above it
+// leaves stretched triangles to single lanes: m = 2, 193 us with 9 and 16, 211
+// with 36, 270 with 120.  Below 16 nothing is gained (m = 1.5, 224 us with 4 to
+// 16).
+//
+// The more a view is magnified, the fewer of its triangles are in sight (two per
+// m x m output pixels and view): a few warps then walk through large boxes while
+// the rest of the chip has nothing to do.  Past kFewInSight they go to the list,
+// which all warps share, where it holds them: 3 x 960x540 into the same size at m
+// = 5 124 -> 101 us, at m = 10 215 -> 96, at m = 20 410 -> 87; 16 x 1920x1080 at
+// m = 20 4735 -> 995.  At m = 4 that gains as often as it loses (16 x 1920x1080
+// 1802 -> 1525, 4 x ERP 4096x2048 into 1920x1080 342 -> 349).  Where the list
+// cannot hold them the pass over the whole mesh shares them out as well, which
+// pays past kShared: 2 x 192x108 into 1920x1080 (m = 10) 237 -> 158 us, 2 x 96x54
+// (m = 20) 463 -> 170, but 2 x 400x225 (m = 4.8) 161 -> 187.
+constexpr float kFewInSight = 4.5f, kShared = 10.f;
+
+int candidate_threshold(const SlotRequest& r) {
+    const float m = magnification(r);
+    if (!(m > kMagnified) || m > kShared) return 4;
+    if (m > kFewInSight) {
+        const RasterDims rd = raster_dims(r.virt, r.params);
+        double in_sight = 0.0;
+        const size_t group = std::min<size_t>(4, r.scene->cams.size());
+        for (size_t v = 0; v < group; ++v) {
+            const rvsb_camera& c = r.scene->cams[v];
+            in_sight += 2.0 * std::min((double)c.width * c.height, (double)rd.w * rd.h / ((double)m * m));
+        }
+        if (in_sight <= 0.75 * (double)needs_of(r.scene, rd.w, rd.h).large) return 4;
+    }
+    const int side = (int)std::max(4.f, std::ceil(m + 1.2f));
     return side * side;
 }
 
@@ -270,7 +294,7 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     D.out_h = virt.height;
     D.precision = p.precision;
     D.small = kRasterVariants[sh.variant].small;
-    if (D.small == 0) D.small = magnified_threshold(magnification(r));
+    if (D.small == 0) D.small = candidate_threshold(r);
     if (rd.rescale) {
         D.rescale = 1;
         D.uv_sx = (float)rd.w / (float)virt.width;
@@ -455,7 +479,7 @@ namespace {
 // Raster variant of a run that is neither pinned nor tuned.  At a magnification
 // of m = 1 a triangle has one or two candidates, and the few above 4 go to the
 // list of large triangles; past m of about 1.1 the threshold follows m
-// (magnified_threshold), so that the ordinary triangles stay with their lanes:
+// (candidate_threshold), so that the ordinary triangles stay with their lanes:
 // 2 x 960x540 into 1920x1080 (m = 2) 158 us against 249 with 4, 8 views of 4
 // ERP 4096x2048 inputs (m = 1.47) 2.06 ms against 2.75, 4 x ERP 4096x2048 into
 // the same 1.67 ms against 1.81.  At m <= 1 a threshold of 16 costs up to 6%
@@ -498,7 +522,7 @@ int BatchCore::tune(const SlotRequest* reqs, int n, cudaStream_t s) {
     // threshold in every slot) take its time.
     constexpr int kRounds = 5;
     bool magnified = false;
-    for (int k = 0; k < n; ++k) magnified = magnified || magnified_threshold(magnification(reqs[k])) != 4;
+    for (int k = 0; k < n; ++k) magnified = magnified || candidate_threshold(reqs[k]) != 4;
     int same[NUM_RASTER_VARIANTS];
     std::vector<int> timed;
     for (int v = 0; v < NUM_RASTER_VARIANTS; ++v) {
@@ -566,13 +590,15 @@ int BatchCore::run(const SlotRequest* reqs, int n, cudaStream_t s, const std::fu
         // The shape the tuner keys on: the batch size bucket and, over the
         // batch, the largest input set and output, the projections and the
         // magnified thresholds (a fixed threshold that suits unmagnified
-        // triangles lists nearly every magnified one).
+        // triangles lists nearly every magnified one; 1: magnified, and all
+        // listed).
         const BatchShape sh = shape_of(reqs, n, 0);
         int proj_in = 0, proj_out = 0, small_lo = INT_MAX, small_hi = 0;
         for (int k = 0; k < n; ++k) {
             proj_in |= 1 << reqs[k].scene->cams[0].projection;
             proj_out |= 1 << reqs[k].virt.projection;
-            const int small = magnified_threshold(magnification(reqs[k]));
+            const int t = candidate_threshold(reqs[k]);
+            const int small = t == 4 && magnification(reqs[k]) > kMagnified ? 1 : t;
             small_lo = std::min(small_lo, small);
             small_hi = std::max(small_hi, small);
         }
