@@ -362,7 +362,10 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     SlotBuffers& B = T.b;
     B.status = ws.status.as<DevStatus>();
     B.large = ws.large.as<uint4>();
-    B.large_capacity = (int)std::min<size_t>(INT32_MAX / 2, ws.large.bytes / sizeof(uint4));
+    // The last of the list's memory holds the huge triangles, two words an entry.
+    const int entries = (int)std::min<size_t>(INT32_MAX / 2, ws.large.bytes / sizeof(uint4));
+    B.huge_capacity = std::min(4096, entries / 32) / 2 * 2;
+    B.large_capacity = entries - B.huge_capacity / 2;
     B.codes = ws.codes.as<uint64_t>();
     B.holes = ws.holes.as<uint32_t>();
     for (int s = 0; s < 4; ++s) B.scan[s] = ws.scan.as<uint64_t>() + (size_t)s * npix;

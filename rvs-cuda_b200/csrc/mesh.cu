@@ -647,6 +647,122 @@ __device__ __forceinline__ bool set_up_entry(const SlotTable& tab, uint4 q, Larg
     return set_up(tab.v[q.y & 255u], tab.t, q.x, !(q.y & 256u), t);
 }
 
+// A triangle of the whole-mesh pass that covers more pixels (about) is huge: its
+// rows go to the warps in kHugeParts parts.  ERP 1024x512 with depth steps into ERP
+// 4096x2048: 2560 us with 65536 and 128 parts, 2070 so, 1972 with 4096 and 16, but
+// noise 480x270 into 3840x2160 1850, 1840 and 2189.
+constexpr int kHugePixels = 16384;
+constexpr int kHugeParts = 32;
+
+// A huge triangle's word: its index, its view, kHugeThere once it is there, and
+// the parts handed out.  One word, so that nothing has to be ordered by a fence: with
+// fences in it, even where they were never reached, the kernel took half as long
+// again over its list (4 x ERP 4096x2048 into ERP 125 -> 194 us).
+constexpr unsigned long long kHugeThere = 1ull << 40, kHugePart = 1ull << 48;
+__device__ __forceinline__ unsigned long long* huge_words(const SlotBuffers& B) {
+    return reinterpret_cast<unsigned long long*>(B.large + B.large_capacity);
+}
+
+// The warp's huge triangles (the lanes `on`) into their words, for all warps to
+// take parts of; returns the lanes whose triangle found none.
+__device__ __forceinline__ unsigned offer_huge(const SlotBuffers& B, uint32_t tri, int view, unsigned on, int lane) {
+    int base = B.huge_capacity;
+    // Words that are all taken are left alone, so that the count stays bounded.
+    if (lane == 0 && *reinterpret_cast<volatile int*>(&B.status->n_huge) < B.huge_capacity)
+        base = atomicAdd(&B.status->n_huge, __popc(on));
+    const int slot = __shfl_sync(0xffffffffu, base, 0) + __popc(on & ((1u << lane) - 1u));
+    const bool in = (on >> lane & 1u) && slot < B.huge_capacity;
+    if (in) atomicExch(huge_words(B) + slot, kHugeThere | (unsigned long long)view << 32 | tri);
+    return on & ~__ballot_sync(0xffffffffu, in);
+}
+
+// Parts of the huge triangles that are there, until all are handed out.  The warp
+// that offered one comes here after it, so none is left over.
+__device__ __forceinline__ void take_huge(const SlotTable& tab, int wid, int lane) {
+    const SlotBuffers& B = tab.b;
+    const int n = min(*reinterpret_cast<volatile int*>(&B.status->n_huge), B.huge_capacity);
+    for (int k = 0; k < n; ++k) {
+        // Not all warps at the same one.
+        unsigned long long* word = huge_words(B) + ((unsigned)wid * 37u + (unsigned)k) % (unsigned)n;
+        for (;;) {
+            unsigned long long h = 0;
+            if (lane == 0) {
+                h = *reinterpret_cast<volatile unsigned long long*>(word);
+                if ((h & kHugeThere) && h / kHugePart < kHugeParts) h = atomicAdd(word, kHugePart);
+            }
+            h = __shfl_sync(0xffffffffu, h, 0);
+            const int part = (int)(h / kHugePart);
+            if (!(h & kHugeThere) || part >= kHugeParts) break;
+            Large t;
+            if (!set_up(tab.v[(int)(h >> 32) & 255], tab.t, (uint32_t)h, false, t)) break;
+            const int rows = (t.s.y1 - t.s.y0 + kHugeParts) / kHugeParts;
+            t.s.y0 += part * rows;
+            t.s.y1 = min(t.s.y1, t.s.y0 + rows - 1);
+            raster_large(t, tab.t.wo, lane);
+        }
+    }
+}
+
+// Every triangle of the views g0 .. g0 + gv - 1: the warps claim groups of quads.
+// Triangles differ much in work, the stretched ones lie together (a row of quads
+// across a depth step, the poles of an equirectangular output), and one can cover
+// most of the output.  Rows of 32 quads dealt out in turn, and each triangle left
+// to the warp that met it, kept the chip waiting for a few warps (18% of the SMs'
+// cycles in use).  So a group is 4 x 4 quads, claimed when a warp is free, the
+// outer rows before the inner, and the huge triangles are shared out: 3 x 1186x198
+// with bars of 6 rows magnified 3.9 times 3968 -> 591 us, 3 x ERP 1024x512 into ERP
+// 4096x2048 with depth steps 4207 -> 1614, with noise 70468 -> 42236, smooth 1213
+// -> 1189; 4 x 1920x1080 with bars 2276 -> 1875, with noise 7062 -> 6345.  Groups
+// of 8 x 4: 595, 2030, 54869, 1076, 1614 and 6191; of 2 x 4: 615, 1666, 33082,
+// 1483, 2400 and 6738.  2 x 480x270 noise into 120x68, whose triangles are all
+// small, pays for it: 119 -> 134.
+//
+// Not inlined: its registers would spill in the list's loops.
+__device__ __noinline__ void whole_mesh(const SlotTable& tab, int g0, int gv, int wid, int nw, int lane) {
+    const DevTarget& T = tab.t;
+    const bool wrap = T.wrap != 0;
+    auto claim = [&] { return lane == 0 ? atomicAdd(&tab.b.status->n_claimed, 1) : 0; };
+    int next = __shfl_sync(0xffffffffu, claim(), 0), first = 0;
+    for (int view = g0; view < min(T.n_views, g0 + gv); ++view) {
+        const DevView& V = tab.v[view];
+        // Fewer rows a group where that leaves some warps without any.
+        int rows = 4;
+        while (rows > 1 && (long long)(V.w - 1) * (V.h - 1) < 4ll * rows * nw) rows /= 2;
+        const int groups = (V.w + 2) / 4, bands = (V.h - 2 + rows) / rows, count = groups * bands;
+        while (next < first + count) {
+            const int g = next - first, claimed = claim();
+            next = __shfl_sync(0xffffffffu, claimed, 0);
+            const int r = g / groups, i0 = (r & 1 ? bands - 1 - r / 2 : r / 2) * rows, j0 = g % groups * 4;
+            if (T.cull && V.erp_cone && tile_culled(V, T, j0 / WARP_TILE, i0 / WARP_TILE)) continue;
+            const int i = i0 + lane / 4, j = j0 + lane % 4;
+            for (int t = 0; t < (wrap ? 4 : 2); ++t) {
+                const uint32_t tri = ((((uint32_t)i << (V.tri_shift - 2)) | (uint32_t)j) << 2) | (uint32_t)t;
+                Large q = {};
+                bool on = lane < 4 * rows && i < V.h - 1 && j < V.w - 1 && (t < 2 || j == 0);
+                if (on) {
+                    // Emission tests of transform.cpp:161-167.
+                    const float4 v01 = __ldg(V.vert + (size_t)i * V.w + j + 1);
+                    const float4 v10 = __ldg(V.vert + (size_t)(i + 1) * V.w + j);
+                    const float4 a = __ldg(V.vert + (size_t)(i + (t & 1)) * V.w + j + (t & 1));
+                    on = v01.z > 0.f && v10.z > 0.f && v01.x > 0.f && v10.x > 0.f &&
+                         (t >= 2 || (a.z > 0.f && a.x > 0.f)) && set_up(V, T, tri, false, q);
+                }
+                const int box = (q.s.x1 - q.s.x0 + 1) * (q.s.y1 - q.s.y0 + 1);
+                const bool medium = on && box <= kMediumPixels;
+                raster_medium(q, medium, T.wo, lane);
+                unsigned m = __ballot_sync(0xffffffffu, on && !medium);
+                // den is twice the triangle's area.
+                const unsigned huge = __ballot_sync(
+                    0xffffffffu, on && box > kHugePixels && q.s.den > 2.f * (float)kHugePixels);
+                if (huge) m = (m & ~huge) | offer_huge(tab.b, tri, view, huge, lane);
+                for (; m; m &= m - 1) raster_large(from_lane(q, __ffs(m) - 1), T.wo, lane);
+            }
+        }
+        first += count;
+    }
+    take_huge(tab, wid, lane);
+}
+
 // Grid (CTAs, slots), LARGE_THREADS threads, over the slot's list.  Medium
 // entries: a warp takes up to 32 consecutive ones (fewer when the list is
 // short, so that all warps have some), sets them up one per lane and
@@ -657,9 +773,9 @@ __device__ __forceinline__ bool set_up_entry(const SlotTable& tab, uint4 q, Larg
 // took 32 in a row kept the kernel waiting: 590 instead of 178 us, ERP to ERP).
 //
 // When the list overflowed (more large triangles than it holds), the warps
-// instead go over all quads of the group's views and
-// rasterise every triangle; those the mesh kernel has done already only
-// repeat keys that are there (atomicMin).
+// instead go over all quads of the group's views (whole_mesh) and rasterise every
+// triangle; those the mesh kernel has done already only repeat keys that are
+// there (atomicMin).
 template <class Tabs>
 __global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
     grid_dep_wait();
@@ -698,50 +814,25 @@ __global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_co
         }
         return;
     }
-    const bool wrap = T.wrap != 0;
-    for (int view = g0; view < min(T.n_views, g0 + gv); ++view) {
-        const DevView& V = tab.v[view];
-        // Quads a warp takes at once: 32, fewer where that leaves some warps
-        // without any, since the listed triangles lie together (a row of quads
-        // across a depth step): 160x90 noise magnified 12 times 698 -> 285
-        // us, 6 x 480x270 with bars of 6 rows 1177 -> 688.  Four groups for
-        // every warp: 289 and 436, but 2 x 480x270 noise into ERP 198 -> 262.
-        int per = 32;
-        while (per > 4 && (long long)((V.w - 1 + per - 1) / per) * (V.h - 1) < nw) per /= 2;
-        const int groups = (V.w - 1 + per - 1) / per;
-        for (long long g = wid; g < (long long)groups * (V.h - 1); g += nw) {
-            const int i = (int)(g / groups), j0 = (int)(g % groups) * per, j = j0 + lane;
-            if (T.cull && V.erp_cone && tile_culled(V, T, j0 / WARP_TILE, i / WARP_TILE)) continue;
-            for (int t = 0; t < (wrap ? 4 : 2); ++t) {
-                const uint32_t tri = ((((uint32_t)i << (V.tri_shift - 2)) | (uint32_t)j) << 2) | (uint32_t)t;
-                Large r = {};
-                bool on = lane < per && j < V.w - 1 && (t < 2 || j == 0);
-                if (on) {
-                    // Emission tests of transform.cpp:161-167.
-                    const float4 v01 = __ldg(V.vert + (size_t)i * V.w + j + 1);
-                    const float4 v10 = __ldg(V.vert + (size_t)(i + 1) * V.w + j);
-                    const float4 a = __ldg(V.vert + (size_t)(i + (t & 1)) * V.w + j + (t & 1));
-                    on = v01.z > 0.f && v10.z > 0.f && v01.x > 0.f && v10.x > 0.f &&
-                         (t >= 2 || (a.z > 0.f && a.x > 0.f)) && set_up(V, T, tri, false, r);
-                }
-                const bool medium = on && (r.s.x1 - r.s.x0 + 1) * (r.s.y1 - r.s.y0 + 1) <= kMediumPixels;
-                raster_medium(r, medium, T.wo, lane);
-                for (unsigned m = __ballot_sync(0xffffffffu, on && !medium); m; m &= m - 1)
-                    raster_large(from_lane(r, __ffs(m) - 1), T.wo, lane);
-            }
-        }
-    }
+    whole_mesh(tab, g0, gv, wid, nw, lane);
 }
 
-// Empty keys in the z-buffers of views g0 .. g0 + gv - 1 of every slot, and
-// an empty list of large triangles.  Grid (CTAs, slots).
+// Empty keys in the z-buffers of views g0 .. g0 + gv - 1 of every slot, an
+// empty list of large triangles and the counters of the pass over the whole mesh.  Grid (CTAs, slots).
 template <class Tabs>
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Tabs tabs, int g0, int gv) {
     grid_dep_wait();
     const SlotTable& tab = tabs.at(blockIdx.y);
     const DevTarget& T = tab.t;
     if (g0 >= T.n_views) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) tab.b.status->n_large = 0;
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) {
+            tab.b.status->n_large = 0;
+            tab.b.status->n_claimed = 0;
+            tab.b.status->n_huge = 0;
+        }
+        for (int k = threadIdx.x; k < tab.b.huge_capacity; k += 256) huge_words(tab.b)[k] = 0ull;
+    }
     const size_t n = (size_t)min(gv, T.n_views - g0) * T.wo * T.ho;
     unsigned long long* z = tab.v[g0].z;  // the group's buffers lie back to back from a 16-byte boundary
     if (blockIdx.x == 0 && threadIdx.x == 0 && (n & 1)) z[n - 1] = kEmptyKey;

@@ -214,7 +214,8 @@ static int unbacked_buffers(const SlotTable& t) {
     int bad = 0;
     auto need = [&](const void* p, size_t bytes) { bad += !backed(p, bytes); };
     need(t.b.status, sizeof(DevStatus));
-    need(t.b.large, sizeof(uint4) * (size_t)t.b.large_capacity);
+    // and the huge triangles after it
+    need(t.b.large, sizeof(uint4) * (size_t)t.b.large_capacity + 8 * (size_t)t.b.huge_capacity);
     need(t.b.codes, 8 * n);
     need(t.b.holes, 4 * (size_t)((t.t.wo + 31) / 32) * t.t.ho);
     for (const uint64_t* p : t.b.scan) need(p, 8 * n);
