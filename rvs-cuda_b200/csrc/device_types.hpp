@@ -81,7 +81,7 @@ struct DevStatus {
     int n_large;        // large triangles entered in the list (may exceed its capacity)
     int n_holes;        // nonzero when some pixel is a hole
     int n_claimed;      // groups of quads claimed by the pass over the whole mesh
-    int n_huge;         // huge triangles it has met (may exceed their slots)
+    int n_huge;         // huge triangles that are shared out (may exceed their words)
 };
 
 // Optional intermediate outputs (device pointers, may be null).
@@ -139,7 +139,7 @@ struct SlotBuffers {
     DevStatus* status;   // 1 entry
     uint4* large;        // large triangles of the view group, `large_capacity` entries
     int large_capacity;
-    int huge_capacity;   // words after the list for the huge triangles the pass over the whole mesh meets
+    int huge_capacity;   // words after the list, one per huge triangle that is shared out
     // Running blend between view groups: (c0, c1) and (c2, weight sum) per
     // pixel; they share the memory of the last scan buffer and the codes,
     // which are written later.

@@ -364,7 +364,7 @@ void BatchCore::fill(SlotTable& T, int k, const SlotRequest& r, const BatchShape
     B.large = ws.large.as<uint4>();
     // The last of the list's memory holds the huge triangles, two words an entry.
     const int entries = (int)std::min<size_t>(INT32_MAX / 2, ws.large.bytes / sizeof(uint4));
-    B.huge_capacity = std::min(4096, entries / 32) / 2 * 2;
+    B.huge_capacity = std::min(8192, entries / 16) / 2 * 2;
     B.large_capacity = entries - B.huge_capacity / 2;
     B.codes = ws.codes.as<uint64_t>();
     B.holes = ws.holes.as<uint32_t>();

@@ -647,8 +647,8 @@ __device__ __forceinline__ bool set_up_entry(const SlotTable& tab, uint4 q, Larg
     return set_up(tab.v[q.y & 255u], tab.t, q.x, !(q.y & 256u), t);
 }
 
-// A triangle of the whole-mesh pass that covers more pixels (about) is huge: its
-// rows go to the warps in kHugeParts parts.  ERP 1024x512 with depth steps into ERP
+// A triangle of the whole-mesh pass, or one the list holds whole, that covers more
+// pixels (about) is huge: its rows go to the warps in kHugeParts parts.  ERP 1024x512 with depth steps into ERP
 // 4096x2048: 2560 us with 65536 and 128 parts, 2070 so, 1972 with 4096 and 16, but
 // noise 480x270 into 3840x2160 1850, 1840 and 2189.
 constexpr int kHugePixels = 16384;
@@ -676,31 +676,43 @@ __device__ __forceinline__ unsigned offer_huge(const SlotBuffers& B, uint32_t tr
     return on & ~__ballot_sync(0xffffffffu, in);
 }
 
-// Parts of the huge triangles that are there, until all are handed out.  The warp
-// that offered one comes here after it, so none is left over.
-__device__ __forceinline__ void take_huge(const SlotTable& tab, int wid, int lane) {
-    const SlotBuffers& B = tab.b;
-    const int n = min(*reinterpret_cast<volatile int*>(&B.status->n_huge), B.huge_capacity);
-    for (int k = 0; k < n; ++k) {
-        // Not all warps at the same one.
-        unsigned long long* word = huge_words(B) + ((unsigned)wid * 37u + (unsigned)k) % (unsigned)n;
+// Parts of the huge triangles that are there, until all are handed out, one of each
+// of 32 words at a time.  The warp that offered one comes here after it, so none is
+// left over.
+__device__ __forceinline__ void take_huge(const SlotTable& tab, int n, int wid, int lane) {
+    const unsigned blocks = (unsigned)(n + 31) / 32u;
+    for (unsigned k = 0; k < blocks; ++k) {
+        // Not all warps at the same words.
+        unsigned long long* words = huge_words(tab.b) + ((unsigned)wid * 37u + k) % blocks * 32u;
+        const int there = min(32, (int)(huge_words(tab.b) + n - words));
         for (;;) {
-            unsigned long long h = 0;
-            if (lane == 0) {
-                h = *reinterpret_cast<volatile unsigned long long*>(word);
-                if ((h & kHugeThere) && h / kHugePart < kHugeParts) h = atomicAdd(word, kHugePart);
+            const unsigned long long h =
+                lane < there ? *reinterpret_cast<volatile unsigned long long*>(words + lane) : 0ull;
+            unsigned m = __ballot_sync(0xffffffffu, (h & kHugeThere) && h / kHugePart < kHugeParts);
+            if (!m) break;
+            for (; m; m &= m - 1) {
+                unsigned long long w = 0;
+                if (lane == 0) w = atomicAdd(words + (__ffs(m) - 1), kHugePart);
+                w = __shfl_sync(0xffffffffu, w, 0);
+                const int part = (int)(w / kHugePart);
+                Large t;
+                if (part >= kHugeParts || !set_up(tab.v[(int)(w >> 32) & 255], tab.t, (uint32_t)w, false, t)) continue;
+                const int rows = (t.s.y1 - t.s.y0 + kHugeParts) / kHugeParts;
+                t.s.y0 += part * rows;
+                t.s.y1 = min(t.s.y1, t.s.y0 + rows - 1);
+                raster_large(t, tab.t.wo, lane);
             }
-            h = __shfl_sync(0xffffffffu, h, 0);
-            const int part = (int)(h / kHugePart);
-            if (!(h & kHugeThere) || part >= kHugeParts) break;
-            Large t;
-            if (!set_up(tab.v[(int)(h >> 32) & 255], tab.t, (uint32_t)h, false, t)) break;
-            const int rows = (t.s.y1 - t.s.y0 + kHugeParts) / kHugeParts;
-            t.s.y0 += part * rows;
-            t.s.y1 = min(t.s.y1, t.s.y0 + rows - 1);
-            raster_large(t, tab.t.wo, lane);
         }
     }
+}
+
+__device__ __forceinline__ int huge_count(const SlotBuffers& B) {
+    return min(*reinterpret_cast<volatile int*>(&B.status->n_huge), B.huge_capacity);
+}
+
+__device__ __forceinline__ bool is_huge(const Large& t) {
+    // den is twice the triangle's area.
+    return (t.s.x1 - t.s.x0 + 1) * (t.s.y1 - t.s.y0 + 1) > kHugePixels && t.s.den > 2.f * (float)kHugePixels;
 }
 
 // Every triangle of the views g0 .. g0 + gv - 1: the warps claim groups of quads.
@@ -711,14 +723,12 @@ __device__ __forceinline__ void take_huge(const SlotTable& tab, int wid, int lan
 // cycles in use).  So a group is 4 x 4 quads, claimed when a warp is free, the
 // outer rows before the inner, and the huge triangles are shared out: 3 x 1186x198
 // with bars of 6 rows magnified 3.9 times 3968 -> 591 us, 3 x ERP 1024x512 into ERP
-// 4096x2048 with depth steps 4207 -> 1614, with noise 70468 -> 42236, smooth 1213
+// 4096x2048 with depth steps 4207 -> 1614, with noise 70468 -> 38292, smooth 1213
 // -> 1189; 4 x 1920x1080 with bars 2276 -> 1875, with noise 7062 -> 6345.  Groups
 // of 8 x 4: 595, 2030, 54869, 1076, 1614 and 6191; of 2 x 4: 615, 1666, 33082,
 // 1483, 2400 and 6738.  2 x 480x270 noise into 120x68, whose triangles are all
 // small, pays for it: 119 -> 134.
-//
-// Not inlined: its registers would spill in the list's loops.
-__device__ __noinline__ void whole_mesh(const SlotTable& tab, int g0, int gv, int wid, int nw, int lane) {
+__device__ __forceinline__ void whole_mesh(const SlotTable& tab, int g0, int gv, int wid, int nw, int lane) {
     const DevTarget& T = tab.t;
     const bool wrap = T.wrap != 0;
     auto claim = [&] { return lane == 0 ? atomicAdd(&tab.b.status->n_claimed, 1) : 0; };
@@ -751,16 +761,20 @@ __device__ __noinline__ void whole_mesh(const SlotTable& tab, int g0, int gv, in
                 const bool medium = on && box <= kMediumPixels;
                 raster_medium(q, medium, T.wo, lane);
                 unsigned m = __ballot_sync(0xffffffffu, on && !medium);
-                // den is twice the triangle's area.
-                const unsigned huge = __ballot_sync(
-                    0xffffffffu, on && box > kHugePixels && q.s.den > 2.f * (float)kHugePixels);
+                const unsigned huge = __ballot_sync(0xffffffffu, on && is_huge(q));
                 if (huge) m = (m & ~huge) | offer_huge(tab.b, tri, view, huge, lane);
                 for (; m; m &= m - 1) raster_large(from_lane(q, __ffs(m) - 1), T.wo, lane);
             }
         }
         first += count;
     }
-    take_huge(tab, wid, lane);
+}
+
+// What the list does not hold.  Not inlined: its registers would spill in the
+// list's loops.
+__device__ __noinline__ void large_rest(const SlotTable& tab, int g0, int gv, bool overflow, int wid, int nw, int lane) {
+    if (overflow) whole_mesh(tab, g0, gv, wid, nw, lane);
+    take_huge(tab, huge_count(tab.b), wid, lane);
 }
 
 // Grid (CTAs, slots), LARGE_THREADS threads, over the slot's list.  Medium
@@ -787,6 +801,7 @@ __global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_co
     const int wid = blockIdx.x * (LARGE_THREADS / 32) + (threadIdx.x >> 5), nw = gridDim.x * (LARGE_THREADS / 32);
     if (n <= tab.b.large_capacity) {
         const uint4* list = tab.b.large;
+        bool offered = false;
         for (int base = 0; base < n; base += 32 * nw) {
             // Lane k looks at the warp's k-th entry of the round.
             const int e = base + lane * nw + wid;
@@ -798,10 +813,22 @@ __global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_co
                 if (set_up_entry(tab,
                                  make_uint4(__shfl_sync(0xffffffffu, q.x, k), __shfl_sync(0xffffffffu, q.y, k),
                                             __shfl_sync(0xffffffffu, q.z, k), __shfl_sync(0xffffffffu, q.w, k)),
-                                 t))
+                                 t)) {
+                    // A triangle wider than 4e4 pixels was entered whole: 6 x ERP
+                    // 796x226 magnified 38 times with bars at arm's length 2278 us
+                    // with such triangles left to one warp each, 341 shared out.
+                    const uint32_t general = __shfl_sync(0xffffffffu, q.y, k);
+                    if ((general & 256u) && is_huge(t)) {
+                        offered = true;
+                        if (!offer_huge(tab.b, t.tri, (int)(general & 255u), 1u, lane)) continue;
+                    }
                     raster_large(t, T.wo, lane);
+                }
             }
         }
+        // One warp in four looks for others' huge triangles (a word that all read
+        // takes their reads in turn), under the loop that follows.
+        const int huge = threadIdx.x < 32 ? huge_count(tab.b) : 0;
         const int per = min(32, (n + nw - 1) / nw);
         for (int e0 = wid * per; e0 < n; e0 += nw * per) {
             Large t = {};
@@ -812,9 +839,9 @@ __global__ void __launch_bounds__(LARGE_THREADS, 8) large_kernel(const __grid_co
             }
             raster_medium(t, on, T.wo, lane);
         }
-        return;
+        if (huge == 0 && !offered) return;
     }
-    whole_mesh(tab, g0, gv, wid, nw, lane);
+    large_rest(tab, g0, gv, n > tab.b.large_capacity, wid, nw, lane);
 }
 
 // Empty keys in the z-buffers of views g0 .. g0 + gv - 1 of every slot, an
@@ -825,14 +852,14 @@ __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Tabs
     const SlotTable& tab = tabs.at(blockIdx.y);
     const DevTarget& T = tab.t;
     if (g0 >= T.n_views) return;
-    if (blockIdx.x == 0) {
-        if (threadIdx.x == 0) {
-            tab.b.status->n_large = 0;
-            tab.b.status->n_claimed = 0;
-            tab.b.status->n_huge = 0;
-        }
-        for (int k = threadIdx.x; k < tab.b.huge_capacity; k += 256) huge_words(tab.b)[k] = 0ull;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        tab.b.status->n_large = 0;
+        tab.b.status->n_claimed = 0;
+        tab.b.status->n_huge = 0;
     }
+    const unsigned some = min(gridDim.x, 32u);
+    if (blockIdx.x < some)
+        for (int k = blockIdx.x * 256 + threadIdx.x; k < tab.b.huge_capacity; k += some * 256) huge_words(tab.b)[k] = 0ull;
     const size_t n = (size_t)min(gv, T.n_views - g0) * T.wo * T.ho;
     unsigned long long* z = tab.v[g0].z;  // the group's buffers lie back to back from a 16-byte boundary
     if (blockIdx.x == 0 && threadIdx.x == 0 && (n & 1)) z[n - 1] = kEmptyKey;

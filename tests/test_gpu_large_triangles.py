@@ -16,13 +16,13 @@ pytestmark = pytest.mark.gpu
 
 THRESHOLD = 4  # candidate pixels of raster variant 0
 BAND = 8192    # pixels of a list entry
-HUGE = 65536   # covered pixels above which the whole-mesh pass shares a triangle out
+HUGE = 16384   # covered pixels above which a triangle is shared out
 
 
 def _capacity(inputs):
     """Entries of the list, and slots for the huge triangles."""
     entries = max(1 << 14, sum(c.width * c.height for c in inputs) // 11)
-    slots = min(4096, entries // 32) // 2 * 2
+    slots = min(8192, entries // 16) // 2 * 2
     return entries - slots // 2, slots
 
 
@@ -124,7 +124,7 @@ def test_noise_overflows_the_list(ctx, w, h, wo, ho):
 @pytest.mark.parametrize("w,h,slots", [(32, 24, "enough"), (64, 48, "too few")])
 def test_huge_triangles_of_a_full_list(ctx, w, h, slots):
     """Noise of few quads over a 3840x2160 view: hundreds of huge triangles among
-    those whose bands overflow the list.  The 512 slots hold the smaller mesh's;
+    those whose bands overflow the list.  The 1,024 words hold the smaller mesh's;
     those of the larger that find none stay with their warps."""
     wl = scenes.random_pose_small(n_views=2, w=w, h=h, seed=370)
     rng = np.random.default_rng(371)
@@ -150,3 +150,19 @@ def test_huge_triangles_across_the_seam(ctx):
     target.position[1] += 0.2
     entries, _, huge = _against_oracle(ctx, wl, target, planes)
     assert entries > 1.1 * _capacity(wl.inputs)[0] and huge > 10, (entries, huge)
+
+
+def test_triangles_wider_than_the_list_knows_boxes_for(ctx):
+    """A camera that has moved in among the points: triangles up to its plane,
+    wider than 40,000 pixels, are listed whole and shared out, the list not
+    full."""
+    wl = scenes.random_pose_small(n_views=2, w=96, h=48, seed=380)
+    rng = np.random.default_rng(381)
+    planes = [(y, u, v, rng.integers(0, 65536, d.shape).astype(np.uint16)) for y, u, v, d in wl.planes]
+    target = copy.deepcopy(wl.targets[0])
+    target.width, target.height = 1280, 720
+    target.principle_point[0], target.principle_point[1] = 640.0, 360.0
+    target.focal[0] = target.focal[1] = 1000.0
+    target.position[0] += 0.5
+    entries, lengths, huge = _against_oracle(ctx, wl, target, planes)
+    assert entries <= _capacity(wl.inputs)[0] and (lengths > 6e4).sum() > 10 and huge > 50, (entries, lengths.max(), huge)
