@@ -146,9 +146,9 @@ struct Tri {
 // overlaps, and one loop runs over the candidates of both (measured with the
 // perspective-only instantiation against one triangle after the other: 164 ->
 // 148 M warp instructions on 4 x 1920x1080 -> 1920x1080, the stage 233 -> 196
-// us, 200 -> 160 us a view in a batch of 8; now 138 M, 164 and 149).  The kernel
-// is bound by instruction issue (87% of cycles); the atomics take no time of their own
-// (without them 191 us).
+// us, 200 -> 160 us a view in a batch of 8).  The kernel, since then 139 M
+// instructions and 164 us, is bound by instruction issue (87% of cycles); the
+// atomics took 5 of the 196 us.
 //
 // Candidate range: a covered pixel's centre lies within the bounding box
 // grown by the tolerance tri_range (device_common.cuh) derives, and
@@ -871,7 +871,8 @@ __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Tabs
 
 // Quad rows per warp, by how many waves of warps (148 SMs x 32) 8 rows each
 // would make.  More rows warp fewer vertices twice (one row of 1 + 1 / rows),
-// fewer leave shorter warps at the end of the launch.  Below 2 waves 4 rows: 2
+// fewer leave shorter warps at the end of the launch (times of the general kernel,
+// before launch_mesh_kernels' instantiations).  Below 2 waves 4 rows: 2
 // x 960x540 43 us the stage, 49 with 8, 61 with 16.  Below 40 waves 8: 4 x
 // 1920x1080 193 us (16 rows: 196), 4 x ERP 4096x2048 into ERP 1076 (16: 1121,
 // 32: 1156).  Above, where the end does not matter, 32: 8 poses of the 1080p
